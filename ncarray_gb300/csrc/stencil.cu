@@ -159,8 +159,7 @@ stencil_tma_kernel(const __grid_constant__ CUtensorMap tmap, T* __restrict__ out
           pm[j] = q;
           pp[j] = q;
         } else if constexpr (MODE == 1) {
-          pm[j] = W.w[4] * v[1][j + 1];
-          pp[j] = W.w[22] * v[1][j + 1];
+          pm[j] = pp[j] = T(0);   // the z terms are added below
           T s = W.w[13] * v[1][j + 1];
           s = fmaT(W.w[12], v[1][j], s);
           s = fmaT(W.w[14], v[1][j + 2], s);
@@ -185,7 +184,8 @@ stencil_tma_kernel(const __grid_constant__ CUtensorMap tmap, T* __restrict__ out
       if (active && i >= 2) {
         T o[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) o[j] = fmaT(W.dt, acc_a[j] + pp[j], cen[j]);
+        for (int j = 0; j < 4; ++j)
+          o[j] = fmaT(W.dt, MODE == 1 ? fmaT(W.w[22], v[1][j + 1], acc_a[j]) : acc_a[j] + pp[j], cen[j]);
         T* dst = out + ((size_t)(p - 1) * ny + y) * nx + x;
         if constexpr (sizeof(T) == 4) {
           *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
@@ -196,7 +196,8 @@ stencil_tma_kernel(const __grid_constant__ CUtensorMap tmap, T* __restrict__ out
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        acc_a[j] = acc_b[j] + p0[j];   // output p: now lacks only plane p+1
+        // output p: now lacks only plane p+1 (star: plane p-1's part is its centre value)
+        acc_a[j] = MODE == 1 ? fmaT(W.w[4], cen[j], p0[j]) : acc_b[j] + p0[j];
         acc_b[j] = pm[j];              // output p+1: plane p's dz=-1 part
         cen[j] = v[1][j + 1];          // centre of output p
       }
@@ -210,6 +211,272 @@ stencil_tma_kernel(const __grid_constant__ CUtensorMap tmap, T* __restrict__ out
   if (timed_out && threadIdx.x == 0) {
     atomicExch(&g_stencil_status, (int)NCA_ERR_TIMEOUT);
     for (int k = i; k < issued; ++k) mbar_wait(bbase + 8 * (k % NST), (uint32_t)((k / NST) & 1), kWaitNs / 2);
+  }
+}
+
+// ---- three Jacobi steps per pass (float32) ------------------------------------------
+// nca_stencil3d_iterate moves the grid through HBM once per step, 8 bytes a
+// point, and the one-step kernel above already runs at 0.97 of the measured
+// copy rate (512^3, 7 points: 163 us a step), so only fewer passes help. This
+// kernel advances three steps while a plane of a tile is on the chip:
+// a CTA of NW warps owns a tile of 128 x (NW * R) columns, halo included, and
+// marches along z. TMA streams the planes into a ring of T3_NST stages; a warp
+// holds R whole 128-column rows (lane l the columns 4l..4l+3), so the x
+// neighbours come from two shuffles and the y neighbours inside a warp from
+// registers; the rows next to a warp's cross shared memory. The three steps of
+// an iteration are independent: step k + 1 takes the plane that step k
+// completed in the iteration before, so one barrier per plane suffices (the
+// exchange is double-buffered by parity). y, z and centre terms are packed
+// float32 pairs, x terms (across the pairs) scalars on their halves: 1071 us
+// for ten steps of 512^3 against 1327 with scalars only (at 16 x 2 rows: 1118).
+// The rolling accumulators add the same terms in the same order as the
+// one-step kernel, so the results equal three single steps bit for bit. Values
+// outside the grid are zeroed after every step (the zero halo); the tile's
+// outer three rows and columns are recomputed by the neighbouring tiles. x
+// tiles advance by 120 columns (480 bytes: boxes start on 16-byte boundaries).
+// Bound: instruction issue (about 10 a point and step with the recomputed halo
+// and the tiles' overhang of 512, 0.55 of the issue slots). Star 14 warps x 3
+// rows, isotropic 12 x 2 (register-bound): ten steps of 512^3 float32 1702 ->
+// 1071 us (7 points), 1700 -> 1615 us (27); (64, 64, 64) 83 -> 53, 103 -> 48;
+// (200, 300, 400) 342 -> 241, 430 -> 351.
+constexpr int T3_K = 3, T3_EX = 128, T3_HX = 4;
+constexpr int T3_TX = T3_EX - 2 * T3_HX;
+constexpr int T3_NST = 4;
+constexpr int T3_LAG = 2 * T3_K + 2;   // iterations from a plane's arrival to the output of the plane 5 below it
+template <int NW, int R>
+struct T3 {   // sizes of a CTA of NW warps
+  static constexpr int EY = NW * R, TY = EY - 2 * T3_K;
+  static constexpr int STAGE = T3_EX * EY * 4;
+  static constexpr int XB = NW * 2 * T3_EX * 4;                        // one exchange buffer
+  static constexpr int SMEM = T3_NST * STAGE + 2 * (T3_K - 1) * XB + T3_NST * 8;
+};
+
+template <int V> struct IntC { static constexpr int value = V; };
+// the step's weights as packed pairs: kernel parameters that the packed
+// instructions read from the constant bank instead of registers
+struct Pairs {
+  float2 dt, z0, z1, c, y0, y1;   // star; isotropic: z0, z1, c, y0 = the weights by distance class 3, 2, 0, 1
+  float x0, x1;
+};
+struct Row4 { float2 a, b; };   // four consecutive columns
+
+__device__ __forceinline__ unsigned long long u2(float2 a) { return *reinterpret_cast<unsigned long long*>(&a); }
+__device__ __forceinline__ float2 f2(unsigned long long a) { return *reinterpret_cast<float2*>(&a); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(u2(a)), "l"(u2(b)), "l"(u2(c)));
+  return f2(d);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(u2(a)), "l"(u2(b)));
+  return f2(d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(u2(a)), "l"(u2(b)));
+  return f2(d);
+}
+__device__ __forceinline__ Row4 row4(float4 m) { return Row4{make_float2(m.x, m.y), make_float2(m.z, m.w)}; }
+__device__ __forceinline__ Row4 zero4() { return Row4{make_float2(0.f, 0.f), make_float2(0.f, 0.f)}; }
+
+// one step's rolling state of a thread's rows: a (the output one plane back,
+// lacking the newest plane), b (isotropic form: the older plane's part of the
+// current output) and c, the centre values of the plane before
+template <int R>
+struct Step3 { Row4 a[R], b[R], c[R]; };
+
+// adds a plane (rows r[0..R-1] with the rows above and below) to a step's
+// state and returns the completed output rows of the plane before
+template <int MODE, int R>
+__device__ __forceinline__ void step_plane(Step3<R>& S, const Row4* r, const Row4& top, const Row4& bot,
+                                           const Pairs& W, Row4* o) {
+  const float2 dt = W.dt;
+  if constexpr (MODE == 1) {
+    const float2 wz0 = W.z0, wz1 = W.z1, wc = W.c, wy0 = W.y0, wy1 = W.y1;
+    const float wx0 = W.x0, wx1 = W.x1;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const Row4 v = r[i];
+      const Row4 up = i == 0 ? top : r[i > 0 ? i - 1 : 0], dn = i == R - 1 ? bot : r[i < R - 1 ? i + 1 : i];
+      const float lf = __shfl_up_sync(0xffffffffu, v.b.y, 1), rt = __shfl_down_sync(0xffffffffu, v.a.x, 1);
+      o[i].a = fma2(dt, fma2(wz1, v.a, S.a[i].a), S.c[i].a);
+      o[i].b = fma2(dt, fma2(wz1, v.b, S.a[i].b), S.c[i].b);
+      float2 sa = mul2(wc, v.a), sb = mul2(wc, v.b);
+      // x neighbours sit across the pairs: scalar FMAs on the halves, no repacking
+      sa = make_float2(__fmaf_rn(wx0, lf, sa.x), __fmaf_rn(wx0, v.a.x, sa.y));
+      sb = make_float2(__fmaf_rn(wx0, v.a.y, sb.x), __fmaf_rn(wx0, v.b.x, sb.y));
+      sa = make_float2(__fmaf_rn(wx1, v.a.y, sa.x), __fmaf_rn(wx1, v.b.x, sa.y));
+      sb = make_float2(__fmaf_rn(wx1, v.b.y, sb.x), __fmaf_rn(wx1, rt, sb.y));
+      sa = fma2(wy0, up.a, sa);
+      sb = fma2(wy0, up.b, sb);
+      sa = fma2(wy1, dn.a, sa);
+      sb = fma2(wy1, dn.b, sb);
+      // the older plane's term: its centre is the value kept for the output
+      S.a[i].a = fma2(wz0, S.c[i].a, sa);
+      S.a[i].b = fma2(wz0, S.c[i].b, sb);
+      S.c[i] = v;
+    }
+  } else {
+    // isotropic: per row the sum of the two x neighbours; F and K as in the one-step kernel
+    auto xsum = [](const Row4& v) {
+      const float lf = __shfl_up_sync(0xffffffffu, v.b.y, 1), rt = __shfl_down_sync(0xffffffffu, v.a.x, 1);
+      return Row4{make_float2(__fadd_rn(lf, v.a.y), __fadd_rn(v.a.x, v.b.x)),
+                  make_float2(__fadd_rn(v.a.y, v.b.y), __fadd_rn(v.b.x, rt))};
+    };
+    const float2 w0 = W.c, w1 = W.y0, w2 = W.z1, w3 = W.z0;
+    Row4 xu = xsum(top), xc = xsum(r[0]);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const Row4 v = r[i];
+      const Row4 up = i == 0 ? top : r[i > 0 ? i - 1 : 0], dn = i == R - 1 ? bot : r[i < R - 1 ? i + 1 : i];
+      const Row4 xd = xsum(dn);
+      const float2 Fa = add2(add2(xc.a, up.a), dn.a), Fb = add2(add2(xc.b, up.b), dn.b);
+      const float2 Ka = add2(xu.a, xd.a), Kb = add2(xu.b, xd.b);
+      const float2 pa = fma2(w2, Ka, fma2(w1, Fa, mul2(w0, v.a))), pb = fma2(w2, Kb, fma2(w1, Fb, mul2(w0, v.b)));
+      const float2 qa = fma2(w3, Ka, fma2(w2, Fa, mul2(w1, v.a))), qb = fma2(w3, Kb, fma2(w2, Fb, mul2(w1, v.b)));
+      o[i].a = fma2(dt, add2(S.a[i].a, qa), S.c[i].a);
+      o[i].b = fma2(dt, add2(S.a[i].b, qb), S.c[i].b);
+      S.a[i].a = add2(S.b[i].a, pa);
+      S.a[i].b = add2(S.b[i].b, pb);
+      S.b[i].a = qa;
+      S.b[i].b = qb;
+      S.c[i] = v;
+      xu = xc;
+      xc = xd;
+    }
+  }
+}
+
+template <int MODE, int NW, int R>
+__global__ void __launch_bounds__(32 * NW, 1)
+stencil_tma3_kernel(const __grid_constant__ CUtensorMap tmap, float* __restrict__ out, int nx, int ny, int nz, int zt,
+                    const __grid_constant__ Pairs W) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  constexpr int EY = T3<NW, R>::EY, STAGE = T3<NW, R>::STAGE, XB = T3<NW, R>::XB;
+  __shared__ volatile int failed;   // a bounded wait ran out
+  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+  unsigned char* const xbuf = smem + T3_NST * STAGE;   // [parity][step][warp][2 rows]
+  const uint32_t bbase = sbase + T3_NST * STAGE + 2 * (T3_K - 1) * XB;
+  const int x0 = blockIdx.x * T3_TX - T3_HX, y0 = blockIdx.y * T3<NW, R>::TY - T3_K, z0 = blockIdx.z * zt;
+  const int zend = min(z0 + zt, nz);
+  const int nin = zend - z0 + 2 * T3_K;       // planes read: z0-3 .. zend+2
+  const int nit = zend - z0 + T3_LAG;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    failed = 0;
+    for (int s = 0; s < T3_NST; ++s)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bbase + 8 * s) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int k = threadIdx.x; k < 2 * (T3_K - 1) * XB / 16; k += 32 * NW)
+    reinterpret_cast<float4*>(xbuf)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();
+  auto issue = [&](int k) {   // input plane k of the march into its stage
+    const uint32_t bar = bbase + 8 * (k % T3_NST);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)STAGE) : "memory");
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(sbase + (k % T3_NST) * STAGE), "l"(reinterpret_cast<unsigned long long>(&tmap)), "r"(x0), "r"(y0),
+        "r"(z0 - T3_K + k), "r"(bar) : "memory");
+  };
+  int issued = 0;
+  if (threadIdx.x == 0)
+    for (; issued < T3_NST && issued < nin; ++issued) issue(issued);
+  Step3<R> S[T3_K];
+  Row4 P[T3_K][R];   // the plane each step takes this iteration
+#pragma unroll
+  for (int k = 0; k < T3_K; ++k)
+#pragma unroll
+    for (int i = 0; i < R; ++i) S[k].a[i] = S[k].b[i] = S[k].c[i] = P[k][i] = zero4();
+  const int gx = x0 + 4 * lane, gy = y0 + warp * R;
+  // rows inside the grid (rin) and rows this thread stores (rout)
+  const bool xin = gx >= 0 && gx < nx;
+  unsigned rin = 0, rout = 0;
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int row = warp * R + i;
+    if (xin && gy + i >= 0 && gy + i < ny) rin |= 1u << i;
+    if (((rin >> i) & 1u) && lane > 0 && lane < 31 && row >= T3_K && row < EY - T3_K) rout |= 1u << i;
+  }
+  const bool inside = x0 >= 0 && x0 + T3_EX <= nx && y0 >= 0 && y0 + EY <= ny;   // no masks in x and y
+  // the rows above and below this warp's in the exchange buffers (a tile's
+  // first and last warp read their own: halo rows whose values are not used)
+  const int above = (warp > 0 ? (warp - 1) * 2 + 1 : 0) * 32 + lane;
+  const int below = (warp < NW - 1 ? (warp + 1) * 2 : warp * 2) * 32 + lane;
+  // one iteration; PAR: its parity. The steps run last to first: a step's old
+  // centre rows are dead when the step before it emits its plane, so over two
+  // iterations (unrolled below) every row stays in the registers it was
+  // computed in.
+  auto iterate = [&](int i, auto PAR) {
+    constexpr int par = decltype(PAR)::value;
+    const int st = i % T3_NST;
+    const bool has = i < nin;
+    const bool ok = !has || mbar_wait(bbase + 8 * st, (uint32_t)((i / T3_NST) & 1), kWaitNs);
+    const float4* xr = reinterpret_cast<const float4*>(xbuf + (par ^ 1) * (T3_K - 1) * XB);
+    float4* xw = reinterpret_cast<float4*>(xbuf + par * (T3_K - 1) * XB) + warp * 64 + lane;
+    // (after the last input plane the stage holds an older one: finite values that no output uses)
+    const float4* plane = reinterpret_cast<const float4*>(smem + st * STAGE) + lane;
+    Row4 top[T3_K], bot[T3_K];
+    auto read = [&](int k) {   // step k's input rows from shared memory
+      if (k > 0) {
+        top[k] = row4(xr[(k - 1) * (XB / 16) + above]);
+        bot[k] = row4(xr[(k - 1) * (XB / 16) + below]);
+        return;
+      }
+      top[0] = row4(plane[(warp > 0 ? warp * R - 1 : 0) * 32]);
+      bot[0] = row4(plane[(warp < NW - 1 ? warp * R + R : warp * R) * 32]);
+#pragma unroll
+      for (int q = 0; q < R; ++q) P[0][q] = row4(plane[(warp * R + q) * 32]);
+    };
+    // the isotropic form has the registers to read everything first (a 512^3
+    // step 162 us against 172); the star form reads per step (107 against 120)
+    if (MODE == 2)
+#pragma unroll
+      for (int k = T3_K - 1; k >= 0; --k) read(k);
+#pragma unroll
+    for (int k = T3_K - 1; k >= 0; --k) {
+      Row4 o[R];
+      if (MODE != 2) read(k);
+      step_plane<MODE, R>(S[k], P[k], top[k], bot[k], W, o);
+      if (k < T3_K - 1) {
+        const int p = z0 - T3_K + i - 1 - 2 * k;   // the plane step k + 1 completed
+        if (p < 0 || p >= nz) {
+          asm volatile("");   // a branch (CTA-uniform), not a select per value
+#pragma unroll
+          for (int q = 0; q < R; ++q) o[q] = zero4();
+        } else if (!inside) {
+          asm volatile("");
+#pragma unroll
+          for (int q = 0; q < R; ++q)
+            if (!((rin >> q) & 1u)) o[q] = zero4();
+        }
+        xw[k * (XB / 16)] = make_float4(o[0].a.x, o[0].a.y, o[0].b.x, o[0].b.y);
+        xw[k * (XB / 16) + 32] = make_float4(o[R - 1].a.x, o[R - 1].a.y, o[R - 1].b.x, o[R - 1].b.y);
+#pragma unroll
+        for (int q = 0; q < R; ++q) P[k + 1][q] = o[q];
+      } else if (i >= T3_LAG && i < nit) {
+        float* dst = out + ((size_t)(z0 + i - T3_LAG) * ny + gy) * nx + gx;
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+          if ((rout >> q) & 1u)
+            *reinterpret_cast<float4*>(dst + (size_t)q * nx) = make_float4(o[q].a.x, o[q].a.y, o[q].b.x, o[q].b.y);
+      }
+    }
+    // the plane's barrier: its stage is read, the exchanged rows are written
+    if (!ok) failed = 1;
+    __syncthreads();
+    if (threadIdx.x == 0 && ok && issued < nin) { issue(issued); ++issued; }
+  };
+  int i = 0;
+#pragma unroll 1
+  for (; i < nit && !failed; i += 2) {   // a wait that ran out ends the march after at most one more plane
+    iterate(i, IntC<0>());
+    iterate(i + 1, IntC<1>());
+  }
+  if (failed && threadIdx.x == 0) {
+    atomicExch(&g_stencil_status, (int)NCA_ERR_TIMEOUT);
+    for (int k = max(0, i - 2); k < issued; ++k) mbar_wait(bbase + 8 * (k % T3_NST), (uint32_t)((k / T3_NST) & 1), kWaitNs / 2);
   }
 }
 
@@ -302,11 +569,12 @@ bool tma_ok(const Grid3& g) {
   return g.nx % 4 == 0 && ((uintptr_t)g.base % 16) == 0 && nca::drv().cuTensorMapEncodeTiled != nullptr;
 }
 
-template <class T, int TX, int TY>
-void encode_map(CUtensorMap* m, const Grid3& g) {
+// tensor map of a grid with boxes of bx x by x 1 points
+template <class T>
+void encode_box(CUtensorMap* m, const Grid3& g, int bx, int by) {
   const cuuint64_t dims[3] = {(cuuint64_t)g.nx, (cuuint64_t)g.ny, (cuuint64_t)g.nz};
   const cuuint64_t strides[2] = {(cuuint64_t)g.nx * sizeof(T), (cuuint64_t)g.nx * g.ny * sizeof(T)};
-  const cuuint32_t box[3] = {(cuuint32_t)box_w<T, TX>(), (cuuint32_t)(TY + 2), 1u};
+  const cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1u};
   const cuuint32_t estr[3] = {1u, 1u, 1u};
   nca::check_cu(nca::drv().cuTensorMapEncodeTiled(
                     m, sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
@@ -318,7 +586,7 @@ void encode_map(CUtensorMap* m, const Grid3& g) {
 template <class T, int TX, int TY>
 void launch_tma(const Grid3& src, const Grid3& dst, const Weights<T>& W, int mode, int zt, cudaStream_t s) {
   CUtensorMap m;
-  encode_map<T, TX, TY>(&m, src);
+  encode_box<T>(&m, src, box_w<T, TX>(), TY + 2);
   dim3 grid((src.nx + TX - 1) / TX, (src.ny + TY - 1) / TY, (src.nz + zt - 1) / zt);
   const size_t smem = NST * stage_bytes<T, TX, TY>() + NST * 8;
   if (mode == 1)
@@ -389,6 +657,44 @@ void launch_one(const Grid3& src, const Grid3& dst, const Weights<T>& W, int mod
   count_launch();
 }
 
+template <int MODE, int NW, int R>
+void launch3_as(const Grid3& src, const Grid3& dst, const Weights<float>& W, cudaStream_t s) {
+  using namespace nca;
+  CUtensorMap m;
+  encode_box<float>(&m, src, T3_EX, T3<NW, R>::EY);
+  const int sms = sm_count(current_device());
+  const int tx = (src.nx + T3_TX - 1) / T3_TX, ty = (src.ny + T3<NW, R>::TY - 1) / T3<NW, R>::TY;
+  // z chunks: one CTA per SM at a time, and every chunk marches 8 planes more
+  // than it stores, so take the split with the fewest planes end to end
+  int64_t best = -1;
+  int zt = src.nz;
+  for (int c = 1; c <= src.nz && c <= 4 * sms; ++c) {
+    const int d = (src.nz + c - 1) / c;
+    const int64_t cost = (((int64_t)tx * ty * ((src.nz + d - 1) / d) + sms - 1) / sms) * (d + T3_LAG + 2);
+    if (best < 0 || cost < best) { best = cost; zt = d; }
+  }
+  auto two = [](float v) { return make_float2(v, v); };
+  Pairs p{};
+  p.dt = two(W.dt);
+  p.c = two(W.w[13]);
+  if (MODE == 1) {
+    p.z0 = two(W.w[4]); p.z1 = two(W.w[22]); p.y0 = two(W.w[10]); p.y1 = two(W.w[16]);
+    p.x0 = W.w[12]; p.x1 = W.w[14];
+  } else {
+    p.y0 = two(W.w[12]); p.z1 = two(W.w[9]); p.z0 = two(W.w[0]);
+  }
+  auto fn = stencil_tma3_kernel<MODE, NW, R>;
+  check_cuda(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, T3<NW, R>::SMEM), "smem attribute");
+  fn<<<dim3(tx, ty, (src.nz + zt - 1) / zt), 32 * NW, T3<NW, R>::SMEM, s>>>(m, (float*)dst.mut, src.nx, src.ny, src.nz, zt, p);
+  check_cuda(cudaGetLastError(), "stencil launch");
+  count_launch();
+}
+
+void launch3(const Grid3& src, const Grid3& dst, const Weights<float>& W, int mode, cudaStream_t s) {
+  if (mode == 1) launch3_as<1, 14, 3>(src, dst, W, s);
+  else launch3_as<2, 12, 2>(src, dst, W, s);
+}
+
 void run(const nca_view* a, const nca_view* b, const double* w27, double dt, int iters, cudaStream_t s) {
   using namespace nca;
   if (!w27) fail(NCA_ERR_INVALID, "null weights");
@@ -400,9 +706,21 @@ void run(const nca_view* a, const nca_view* b, const double* w27, double dt, int
   const char *pa = (const char*)ga.base, *pb = (const char*)gb.base;
   if (pa < pb + bytes && pb < pa + bytes) fail(NCA_ERR_INVALID, "stencil source and destination overlap");
   const int mode = star7(w27) ? 1 : isotropic27(w27) ? 2 : 0;
-  for (int it = 0; it < iters; ++it) {
-    const Grid3& src = (it % 2 == 0) ? ga : gb;
-    const Grid3& dst = (it % 2 == 0) ? gb : ga;
+  // steps 1 .. iters-1 three at a time where the three-step kernel applies
+  // (each pass moves the result to the other grid, and three single steps do
+  // too); the last step runs alone, so that afterwards the two grids hold the
+  // last two iterates, as when every step runs alone
+  const bool three = ga.dtype == NCA_FLOAT32 && mode != 0 && tma_ok(ga) && tma_ok(gb);
+  bool from_a = true;
+  for (int it = 0; it < iters; from_a = !from_a) {
+    const Grid3& src = from_a ? ga : gb;
+    const Grid3& dst = from_a ? gb : ga;
+    if (three && iters - 1 - it >= T3_K) {
+      launch3(src, dst, make_weights<float>(w27, dt), mode, s);
+      it += T3_K;
+      continue;
+    }
+    ++it;
     if (ga.dtype == NCA_FLOAT32) launch_one<float>(src, dst, make_weights<float>(w27, dt), mode, s);
     else launch_one<double>(src, dst, make_weights<double>(w27, dt), mode, s);
   }
