@@ -361,6 +361,11 @@ struct Spec {
   uint32_t ptrmask = 0;   // operands on a pointer axis (kinds 2, 3, 4)
   int lastcta = 0;   // kinds 3 (block teams) and 4: the last CTA over a set of kept positions merges their partials
   int block = 256;   // kinds 1, 2: threads per block (NCA_LB)
+  // kind 2, row segments: vector groups per thread (0: one group per thread), the
+  // dim walked with hoisted operands (-1: none), its indices per warp, the
+  // operands that do not move along it
+  int rowu = 0, loopd = -1, loopf = 1;
+  uint32_t invmask = 0;
   int k4r = 0;       // kind 4: row lanes per warp (row-lane form, one reduced dim rd); 0: thread per column group
   int rd = 0;
   int k4p = 0;       // kind 4 row-lane form on a persistent grid (equal contiguous ranges of units)
@@ -636,6 +641,8 @@ static std::string gen_source(const Spec& sp, const Tape& t) {
      << "\n#define NCA_HAS_SUM " << (sp.has_sum ? 1 : 0) << "\n#define NCA_HAS_MAX " << (sp.has_max ? 1 : 0)
      << "\n#define NCA_HAS_MIN " << (sp.has_min ? 1 : 0) << "\n#define NCA_LASTCTA " << sp.lastcta
      << "\n#define NCA_K4R " << sp.k4r << "\n#define NCA_RD " << sp.rd << "\n#define NCA_K4P " << sp.k4p
+     << "\n#define NCA_ROWU " << sp.rowu << "\n#define NCA_LOOPD " << sp.loopd << "\n#define NCA_LOOPF " << sp.loopf
+     << "\n#define NCA_INVMASK " << sp.invmask << "u\n#define NCA_OUT_ES " << (sp.has_out ? dtinfo(sp.out_dtype).size : 1)
      << "\n#define NCA_K4B " << sp.k4b << "\n#define NCA_K3RV " << sp.k3rv << "\n#define NCA_K3TU " << sp.k3tu << "\n";
   int sum_mode = 1;
   if (sp.nred > 0) {
@@ -692,8 +699,9 @@ static std::string gen_source(const Spec& sp, const Tape& t) {
     const int sz = dtinfo(dt).size;
     return "(nca_w)(" + from_bits(dt, "*(const " + storage_uint(sz) + "*)(" + ptr + ")") + ")";
   };
-  std::ostringstream g, g1;
+  std::ostringstream g_inv, g_var, g1;
   for (int k = 0; k < sp.nops; ++k) {
+    std::ostringstream& g = ((sp.invmask >> k) & 1u) ? g_inv : g_var;
     const int dt = sp.op_dtypes[k];
     const int es = dtinfo(dt).size;
     const std::string base = "OPB_(" + std::to_string(k) + ") + off[" + std::to_string(k) + "]";
@@ -750,8 +758,13 @@ static std::string gen_source(const Spec& sp, const Tape& t) {
   }
   // the kernels take `const NcaArgs A`; the helpers take it by reference
   os << "struct NcaArgs { u64 w[" << L.nwords << "]; };\n";
-  os << "__device__ __forceinline__ void nca_gather(const NcaArgs& A, const i64* off, nca_w (*v)[NCA_VEC]) {\n"
-     << g.str() << "}\n";
+  os << "__device__ __forceinline__ void nca_gather_var(const NcaArgs& A, const i64* off, nca_w (*v)[NCA_VEC]) {\n"
+     << g_var.str() << "}\n";
+  if (sp.invmask)
+    os << "__device__ __forceinline__ void nca_gather_inv(const NcaArgs& A, const i64* off, nca_w (*v)[NCA_VEC]) {\n"
+       << g_inv.str() << "}\n";
+  else
+    os << "#define nca_gather nca_gather_var\n";
   os << "__device__ __forceinline__ void nca_gather1(const NcaArgs& A, const i64* off, nca_w (*v)[NCA_VEC]) {\n"
      << g1.str() << "}\n";
   os << "#define nca_gather_ns nca_gather\n";
@@ -782,6 +795,16 @@ static std::string gen_source(const Spec& sp, const Tape& t) {
     os << "__device__ __forceinline__ constexpr int nca_k4b_opoff(int k) {\n" << of_f.str() << "  return 0;\n}\n";
     os << "__device__ __forceinline__ void nca_sgather(const unsigned char* const* p, nca_w (*v)[NCA_VEC]) {\n"
        << sg.str() << "}\n";
+  }
+  // stride of operand k along the innermost dim, a constant where the mode fixes it
+  if (sp.rowu > 0) {
+    os << "__device__ __forceinline__ i64 nca_ist(const NcaArgs& A, int k) {\n";
+    for (int k = 0; k < sp.nops; ++k) {
+      const int es = dtinfo(sp.op_dtypes[k]).size, m = sp.op_modes[k];
+      if (m == M_CONST || m == M_CONTIG || m == M_PAIR0 || m == M_PAIR1)
+        os << "  if (k == " << k << ") return " << (m == M_CONST ? 0 : m == M_CONTIG ? es : 2 * es) << ";\n";
+    }
+    os << "  return OPS_(k, " << sp.nd - 1 << ");\n}\n";
   }
   // operands whose byte offsets equal an earlier operand's (same strides)
   os << "__device__ __forceinline__ constexpr int nca_sal(int k) {\n  return ";
@@ -1136,6 +1159,7 @@ static std::string plan_key(const Spec& sp, const Tape& t) {
   add(sp.rb); add(sp.tmask); add(sp.tile_bytes); add(sp.unroll); add(sp.qxp); add(sp.minb); add(sp.grp);
   add(sp.ns); add(sp.ld); add(sp.npc); add(sp.ltp8); add(sp.pmask); add(sp.umask); add(sp.nmaps); add(sp.uumask); add(sp.ptrmask);
   add(sp.nob); add(sp.lastcta); add(sp.block); add(sp.k4r); add(sp.rd); add(sp.k4p); add(sp.k3u);
+  add(sp.rowu); add(sp.loopd); add(sp.loopf); add(sp.invmask);
   add(sp.k4b); add(sp.k4b_rb); add(sp.k4b_ns); add(sp.k4b_cb); add(sp.k3rv); add(sp.k3tu);
   k += literal_key(t) + '|';
   add(sp.xvec);
@@ -1191,10 +1215,13 @@ static void compute_magic(int64_t d, uint64_t& word) {
   word = (uint64_t)(uint32_t)m | ((uint64_t)sh << 32);
 }
 
+static int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
 static bool aligned(const void* p, int64_t a) { return a <= 1 || ((uintptr_t)p % (uintptr_t)a) == 0; }
 
 // chooses NCA_VEC and operand modes for a vector axis (the innermost canonical dim)
-static void plan_vec(const Space& s, Spec& sp, int max_vec_elems, bool with_out) {
+// (tail: the kernel handles a last group of fewer elements)
+static void plan_vec(const Space& s, Spec& sp, int max_vec_elems, bool with_out, bool tail = false) {
   const int ax = s.nd - 1;
   int maxsz = 1;
   if (with_out) maxsz = std::max(maxsz, dtinfo(s.out.dtype).size);
@@ -1209,7 +1236,7 @@ static void plan_vec(const Space& s, Spec& sp, int max_vec_elems, bool with_out)
     for (int d = 0; d < ax; ++d) if (s.out.st[d] % (v * isz) != 0) return false;
     return true;
   };
-  while (vec > 1 && (s.shape[ax] % vec != 0 || !out_ok(vec))) vec >>= 1;
+  while (vec > 1 && ((!tail && s.shape[ax] % vec != 0) || !out_ok(vec))) vec >>= 1;
   // a table axis innermost: every lane reads its own panel pointer
   for (int k = 0; k < sp.nops; ++k) if (s.ops[k].ptr && s.ops[k].pts[ax] != 0) vec = 1;
   sp.vec = vec;
@@ -1271,6 +1298,65 @@ static void plan_pairs(const Space& s, Spec& sp) {
       if (same) { sp.op_alias[k] = j; break; }
     }
   }
+}
+
+// kind 2 on row segments (see the kernel): for rows that keep at least 0.6 of a
+// warp's lanes busy, when a thread gets more than one group: U groups of a row
+// and, when some operands stay put along another dim, F indices of that dim per
+// thread, within about 48 registers of operands and with 32 warps per SM left.
+// Measured (us, one group per thread -> segments): (raw - dark) * gain over
+// (96, 512, 1024) uint16 frames 53.8 -> 50.9, over a crop of 500 x 1000 from
+// column 3 76.3 -> 55.7 (82.7 without F), of 509 x 1015 141.6 -> 62.5 (80.3);
+// (65536, 1000) bfloat16 times a row 67.7 -> 63.9 (70.4 without F); x * r + c
+// over (4096, 4096) float32 24.8 -> 22.2, over 4001 x 4001 44.3 -> 23.9. Groups
+// of 16 bytes: two per thread (three and more 2-5 % slower). float64 vectors
+// stay on one group per thread: their arithmetic, not the loads, is the longer
+// part, and batching the loads ends its overlap ((256, 256, 256) times a
+// broadcast plane 45.3 against 47.6).
+static void plan_rows(const Space& s, Spec& sp, int sms) {
+  const int ax = s.nd - 1;
+  sp.rowu = 0; sp.loopd = -1; sp.loopf = 1; sp.invmask = 0;
+  if (!sp.idx32 || s.out.st[ax] != dtinfo(s.out.dtype).size || (sp.w == NCA_FLOAT64 && sp.vec > 1)) return;
+  for (int k = 0; k < sp.nops; ++k) if (s.ops[k].ptr && s.ops[k].pts[ax] != 0) return;
+  const int64_t gi = s.shape[ax] / sp.vec, rows = s.total() / std::max<int64_t>(s.shape[ax], 1);
+  const int wr = std::max(1, dtinfo(sp.w).size / 4) * sp.vec;   // registers of a loaded group
+  bool plain = sp.ptrmask == 0;
+  for (int k = 0; k < sp.nops; ++k) {
+    if (sp.op_modes[k] == M_PAIR0 || sp.op_modes[k] == M_PAIR1) plain = false;   // windows shared between operands
+    // unaligned operands are read element by element: one element a lane is the coalesced form
+    if (sp.op_modes[k] == M_STRIDED && sp.vec == 1 && s.ops[k].st[ax] == dtinfo(s.ops[k].dtype).size && !s.ops[k].ptr)
+      sp.op_modes[k] = M_CONTIG;
+  }
+  // the dim along which the most operands stay put
+  int ninv = 0;
+  for (int d = 0; d < ax && plain; ++d) {
+    if (s.shape[d] < 4) continue;
+    uint32_t m = 0;
+    for (int k = 0; k < sp.nops; ++k) if (s.ops[k].st[d] == 0 && sp.op_modes[k] != M_CONST) m |= 1u << k;
+    const int c = __builtin_popcount(m);
+    if (c > ninv && c < sp.nops) { ninv = c; sp.loopd = d; sp.invmask = m; }
+  }
+  const int nvar = sp.nops - ninv;
+  const int64_t want = (int64_t)sms * 32;   // warps
+  double best = 0.0;
+  for (int u : {8, 4, 2, 1}) {
+    const int64_t nseg = cdiv(gi, 32 * u);
+    const double busy = (double)gi / (double)(nseg * 32 * u);
+    if (u > 1 && (u * wr * std::max(1, sp.nops) > 48 || (wr >= 4 && u > 2) || rows * nseg < want)) continue;
+    if (busy > best + 0.05) { best = busy; sp.rowu = u; }
+  }
+  if (best < 0.6) { sp.rowu = 0; sp.loopd = -1; sp.invmask = 0; return; }
+  if (sp.loopd >= 0) {
+    const int64_t nseg = cdiv(gi, 32 * sp.rowu);
+    for (int f : {8, 4, 2}) {
+      if (f > s.shape[sp.loopd] || f * sp.rowu * wr * nvar > 32) continue;
+      if (rows / s.shape[sp.loopd] * cdiv(s.shape[sp.loopd], f) * nseg < want) continue;
+      sp.loopf = f;
+      break;
+    }
+  }
+  if (sp.loopf == 1) { sp.loopd = -1; sp.invmask = 0; }
+  if (sp.rowu * sp.loopf == 1) sp.rowu = 0;
 }
 
 // The device int that JIT kernels set when a bounded wait gives up (a
@@ -1363,8 +1449,6 @@ static bool rerun_safe(const nca_view* ops, int nops, const nca_view* outs, int 
   }
   return true;
 }
-
-static int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 static void check_broadcast(const int64_t* lshape, int n, const nca_view& v, const char* what) {
   if (v.ndim > n) fail(NCA_ERR_SHAPE, "%s has %d dims, more than the result's %d", what, v.ndim, n);
@@ -1767,9 +1851,10 @@ void expr_eval(const Tape& tape, const nca_view* ops, int nops, const nca_view& 
   bool flat = s.nd == 1 && s.out.st[0] == dtinfo(out.dtype).size && sp.ptrmask == 0;
   for (int k = 0; k < nops && flat; ++k)
     if (s.ops[k].st[0] != 0 && s.ops[k].st[0] != dtinfo(ops[k].dtype).size) flat = false;
-  plan_vec(s, sp, 16, true);
+  plan_vec(s, sp, 16, true, flat);
   if (flat) {
     for (int k = 0; k < nops; ++k) if (sp.op_modes[k] == M_STRIDED && sp.vec > 1) flat = false;
+    if (!flat) plan_vec(s, sp, 16, true);
   }
   sp.kind = flat ? 1 : 2;
   if (sp.kind == 2) {
@@ -1790,16 +1875,32 @@ void expr_eval(const Tape& tape, const nca_view* ops, int nops, const nca_view& 
   bool small_dims = true;
   for (int d = 0; d < s.nd; ++d) if (s.shape[d] >= (1ll << 31)) small_dims = false;
   sp.idx32 = (total / sp.vec < (1ll << 31) && small_dims) ? 1 : 0;
+  const int dev = current_device();
+  if (sp.kind == 2) plan_rows(s, sp, sm_count(dev));
   const WordLayout L = word_layout(sp.nops, sp.nd, sp.nscal, 0, sp.ptrmask != 0);
   std::vector<uint64_t> w;
   fill_common_words(s, sp, tape, L, w);
-  for (int d = 0; d < s.nd; ++d) {
-    int64_t dv = s.shape[d];
-    if (d == s.nd - 1) dv /= sp.vec;
-    compute_magic(dv, w[L.magic + d]);
+  int64_t groups = total / sp.vec;
+  if (sp.rowu > 0) {
+    // units of work: row segments, loopf indices of the loop dim at a time
+    const int64_t nseg = cdiv(s.shape[s.nd - 1] / sp.vec, 32 * sp.rowu);
+    int64_t units = nseg;
+    compute_magic(nseg, w[L.magic + s.nd - 1]);
+    for (int d = 0; d < s.nd - 1; ++d) {
+      const int64_t e = d == sp.loopd ? cdiv(s.shape[d], sp.loopf) : s.shape[d];
+      compute_magic(e, w[L.magic + d]);
+      units *= e;
+    }
+    w[L.nsplit] = (uint64_t)nseg;
+    w[L.chunk] = (uint64_t)units;
+    groups = units * 32;   // threads
+  } else {
+    for (int d = 0; d < s.nd; ++d) {
+      int64_t dv = s.shape[d];
+      if (d == s.nd - 1) dv /= sp.vec;
+      compute_magic(dv, w[L.magic + d]);
+    }
   }
-  const int dev = current_device();
-  const int64_t groups = total / sp.vec;
   // schedule: threads per block, vector groups per thread per trip (kind 1)
   // and resident threads per SM the grid is capped at; the autotuner's
   // cached choice for this (kind, dtypes, operand count, vector width, size
@@ -2523,6 +2624,22 @@ int jit_selftest(const char* arch) {
     sp.op_salias = {-1, -1, -1};
     nvrtc_compile(gen_source(sp, t), a);
     ++n;
+  }
+  // kind 2 on row segments: plain, with a hoisting loop dim (operand 0 stays put along it), pointer operand
+  for (int di : {1, 3}) {
+    auto& d = dts[di];
+    Spec sp;
+    sp.kind = 2; sp.nops = 3; sp.nd = 3; sp.vec = 1; sp.idx32 = 1; sp.w = d[0]; sp.r = d[1]; sp.out_dtype = d[1]; sp.nscal = 1;
+    sp.has_out = true;
+    t.compute_dtype = d[0]; t.result_dtype = d[1];
+    sp.op_dtypes = {d[2], d[2], d[2]}; sp.op_modes = {M_CONTIG, M_CONST, M_CONTIG}; sp.op_salias = {-1, -1, -1};
+    sp.rowu = 4;
+    nvrtc_compile(gen_source(sp, t), a);
+    sp.loopd = 0; sp.loopf = 4; sp.invmask = 1u;
+    nvrtc_compile(gen_source(sp, t), a);
+    sp.loopd = -1; sp.loopf = 1; sp.invmask = 0; sp.ptrmask = 4u; sp.vec = std::min(d[3], 4); sp.op_modes[2] = M_STRIDED;
+    nvrtc_compile(gen_source(sp, t), a);
+    n += 3;
   }
   n += batch_expr_selftest(a.c_str());
   n += stencil_tile_selftest(a.c_str());
