@@ -11,7 +11,8 @@
 //     (__match_any_sync), sums each group by pointer jumping over the group's
 //     lanes and lets one lane per group issue the atomic (warp-aggregated
 //     atomics: the hot bins of skewed index distributions cost one atomic per
-//     warp instead of one per element);
+//     warp instead of one per element), in the common case below only while
+//     the indices do repeat;
 //   - privatises the destination in shared memory when it is small next to the
 //     input (each CTA accumulates its grid-stride share there and adds the
 //     non-zero entries to the destination once);
@@ -33,7 +34,7 @@
 namespace {
 
 constexpr int THREADS = 256;
-constexpr int SMEM_MAX_BYTES = 48 * 1024;   // privatised destination limit per CTA
+constexpr int SMEM_MAX_BYTES = 200 * 1024;  // privatised destination limit per CTA
 
 struct ScatterArgs {
   const char* idx;
@@ -134,16 +135,17 @@ __device__ __forceinline__ void offsets_of(const ScatterArgs& a, long long i, lo
 
 // One grid-stride pass; SMEM: accumulate into the CTA's shared copy of dest.
 template <class D, bool SMEM>
-__global__ void __launch_bounds__(THREADS) scatter_add_kernel(ScatterArgs a) {
+__global__ void __launch_bounds__(SMEM ? 1024 : THREADS) scatter_add_kernel(ScatterArgs a) {
+  const int nthr = SMEM ? (int)blockDim.x : THREADS;
   extern __shared__ __align__(16) unsigned char sm_raw[];
   D* priv = reinterpret_cast<D*>(sm_raw);
   if (SMEM) {
-    for (long long b = threadIdx.x; b < a.dest_n; b += THREADS) priv[b] = D(0);
+    for (long long b = threadIdx.x; b < a.dest_n; b += nthr) priv[b] = D(0);
     __syncthreads();
   }
-  const long long stride = (long long)gridDim.x * THREADS;
+  const long long stride = (long long)gridDim.x * nthr;
   // every lane of a warp runs the same number of rounds (the group sum needs all 32)
-  const long long warp0 = (long long)blockIdx.x * THREADS + (threadIdx.x & ~31);
+  const long long warp0 = (long long)blockIdx.x * nthr + (threadIdx.x & ~31);
   for (long long base = warp0; base < a.n; base += stride) {
     const long long i = base + (threadIdx.x & 31);
     long long t = -1;
@@ -164,7 +166,7 @@ __global__ void __launch_bounds__(THREADS) scatter_add_kernel(ScatterArgs a) {
   }
   if (SMEM) {
     __syncthreads();
-    for (long long b = threadIdx.x; b < a.dest_n; b += THREADS) {
+    for (long long b = threadIdx.x; b < a.dest_n; b += nthr) {
       const D v = priv[b];
       if (v != D(0)) atomic_add<D>(reinterpret_cast<D*>(a.dest + b * a.dest_stride), v);
     }
@@ -180,19 +182,30 @@ __global__ void __launch_bounds__(THREADS) scatter_add_kernel(ScatterArgs a) {
 constexpr int U = 4;
 
 template <class D, class IW, bool SMEM>
-__global__ void __launch_bounds__(THREADS) scatter_fast_kernel(ScatterArgs a, int idx_signed) {
+__global__ void __launch_bounds__(SMEM ? 1024 : THREADS) scatter_fast_kernel(ScatterArgs a, int idx_signed) {
+  const int nthr = SMEM ? (int)blockDim.x : THREADS;
   extern __shared__ __align__(16) unsigned char sm_raw[];
   D* priv = reinterpret_cast<D*>(sm_raw);
   if (SMEM) {
-    for (long long b = threadIdx.x; b < a.dest_n; b += THREADS) priv[b] = D(0);
+    for (long long b = threadIdx.x; b < a.dest_n; b += nthr) priv[b] = D(0);
     __syncthreads();
   }
   const IW* idx = reinterpret_cast<const IW*>(a.idx);
   const D* src = reinterpret_cast<const D*>(a.src);
   const long long ist = a.istr[0] / (long long)sizeof(IW), sst = a.sstr[0] / (long long)sizeof(D);
   const int lane = threadIdx.x & 31;
-  const long long stride = (long long)gridDim.x * THREADS * U;
-  for (long long base = ((long long)blockIdx.x * THREADS + (threadIdx.x & ~31)) * U; base < a.n; base += stride) {
+  const long long stride = (long long)gridDim.x * nthr * U;
+  // Grouping a warp's equal indices costs about 75 clocks per SM and 32
+  // elements, more than the atomics of distinct ones, so a warp groups one trip
+  // in 16 and the others only when 5 lanes of that trip held an element whose
+  // index repeats in its load (an index that takes 7 % of the elements). 2^26 float32 elements, us before -> now: into 2^20
+  // entries 527 -> 367 (L2 atomics, 183 G/s), 12000 528 -> 163 and 50000 527 ->
+  // 165 (private copies, shared-memory atomics); a skewed power law is grouped
+  // as before (2^24: 1205 us), sorted indices too (16 repeats each, 60.5 -> 65:
+  // the price of the choice).
+  bool group = true;
+  int trip = 0;
+  for (long long base = ((long long)blockIdx.x * nthr + (threadIdx.x & ~31)) * U; base < a.n; base += stride, ++trip) {
     IW raw[U];
     D v[U];
 #pragma unroll
@@ -205,19 +218,34 @@ __global__ void __launch_bounds__(THREADS) scatter_fast_kernel(ScatterArgs a, in
         v[k] = src[i * sst];
       }
     }
+    long long t[U];
 #pragma unroll
     for (int k = 0; k < U; ++k) {
-      long long t;
-      if (sizeof(IW) == 4) t = idx_signed ? (long long)(int)(unsigned)raw[k] : (long long)(unsigned)raw[k];
-      else t = (long long)(unsigned long long)raw[k];   // uint64 >= 2^63 reads negative: dropped
-      if (base + k * 32 + lane >= a.n) t = -1;
-      const bool ok = t >= 0 && t < a.dest_n;
-      const unsigned key = ok ? (unsigned)t : 0x80000000u + (unsigned)lane;   // invalid lanes stay alone
+      if (sizeof(IW) == 4) t[k] = idx_signed ? (long long)(int)(unsigned)raw[k] : (long long)(unsigned)raw[k];
+      else t[k] = (long long)(unsigned long long)raw[k];   // uint64 >= 2^63 reads negative: dropped
+      if (base + k * 32 + lane >= a.n || t[k] >= a.dest_n) t[k] = -1;
+    }
+    auto put = [&](int k, D s) {
+      if (SMEM) atomic_add<D>(priv + t[k], s);
+      else atomic_add<D>(reinterpret_cast<D*>(a.dest + t[k] * a.dest_stride), s);
+    };
+    if (!group && (trip & 15) != 0) {
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        if (t[k] >= 0) put(k, v[k]);
+      continue;
+    }
+    bool repeated = false;
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const bool ok = t[k] >= 0;
+      const unsigned key = ok ? (unsigned)t[k] : 0x80000000u + (unsigned)lane;   // invalid lanes stay alone
       const unsigned peers = __match_any_sync(0xffffffffu, key);
       D s = ok ? v[k] : D(0);
       const unsigned above = peers & ~((2u << lane) - 1u);
       int next = above ? __ffs(above) - 1 : lane;
       bool has = above != 0;
+      repeated |= has;
       if (__any_sync(0xffffffffu, has)) {
 #pragma unroll
         for (int r = 0; r < 5; ++r) {
@@ -227,15 +255,13 @@ __global__ void __launch_bounds__(THREADS) scatter_fast_kernel(ScatterArgs a, in
           if (has) { s += ov; next = onext; has = ohas; }
         }
       }
-      if (ok && (peers & ((1u << lane) - 1u)) == 0) {
-        if (SMEM) atomic_add<D>(priv + t, s);
-        else atomic_add<D>(reinterpret_cast<D*>(a.dest + t * a.dest_stride), s);
-      }
+      if (ok && (peers & ((1u << lane) - 1u)) == 0) put(k, s);
     }
+    if ((trip & 15) == 0) group = __popc(__ballot_sync(0xffffffffu, repeated)) >= 5;
   }
   if (SMEM) {
     __syncthreads();
-    for (long long b = threadIdx.x; b < a.dest_n; b += THREADS) {
+    for (long long b = threadIdx.x; b < a.dest_n; b += nthr) {
       const D v = priv[b];
       if (v != D(0)) atomic_add<D>(reinterpret_cast<D*>(a.dest + b * a.dest_stride), v);
     }
@@ -259,21 +285,33 @@ void launch(ScatterArgs& a, cudaStream_t s) {
   const int sms = nca::sm_count(dev);
   const long long bytes = a.dest_n * (long long)sizeof(D);
   long long blocks = (a.n + THREADS - 1) / THREADS;
-  // privatise when the destination fits and every CTA has several times more
-  // elements to add than destination entries to flush
-  const long long priv_ctas = (long long)sms * 4;
-  const bool smem = bytes <= SMEM_MAX_BYTES && a.n >= 4 * priv_ctas * a.dest_n;
+  // privatise when the destination fits and an element comes per two entries that
+  // the CTAs flush (coalesced atomics, about a tenth of a scattered one each): 4
+  // CTAs of 256 threads per SM up to 48 KB, 2 of 512 up to 100 KB, else 1 of
+  // 1024. 2^23 float32 elements into 6000 entries 242 -> 34 us, 25000 75 -> 30,
+  // 50000 69 -> 32; 2^20 into 6000 34 -> 16; 2^23 float64 into 12000 81 -> 46
+  auto pays = [&](int per_sm) { return 2 * a.n >= (long long)sms * per_sm * a.dest_n; };
+  const int pct = bytes <= 48 * 1024 && pays(4) ? 4 : bytes <= 100 * 1024 && pays(2) ? 2 : 1;
+  const int pthreads = 1024 / pct;
+  const long long priv_ctas = (long long)sms * pct;
+  const bool smem = bytes <= SMEM_MAX_BYTES && pays(pct);
   const int isz = (a.idx_dt == NCA_INT64 || a.idx_dt == NCA_UINT64) ? 8 : 4;
   const bool fast = a.nd == 1 && same_src<D>(a.src_dt) && a.dest_n < (1ll << 31) &&
                     a.istr[0] % isz == 0 && a.sstr[0] % (long long)sizeof(D) == 0 &&
                     (uintptr_t)a.idx % isz == 0 && (uintptr_t)a.src % sizeof(D) == 0;
+  auto big = [&](const void* fn) {   // more shared memory than the default limit
+    if (bytes > 48 * 1024)
+      nca::check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "smem attribute");
+  };
   if (fast) {
     const int sgn = a.idx_dt == NCA_INT32 ? 1 : 0;
     long long fb = (a.n + (long long)THREADS * U - 1) / ((long long)THREADS * U);
     if (smem) {
       fb = std::min(fb, priv_ctas);
-      if (isz == 4) scatter_fast_kernel<D, unsigned, true><<<(unsigned)fb, THREADS, (size_t)bytes, s>>>(a, sgn);
-      else scatter_fast_kernel<D, unsigned long long, true><<<(unsigned)fb, THREADS, (size_t)bytes, s>>>(a, sgn);
+      big(isz == 4 ? (const void*)scatter_fast_kernel<D, unsigned, true>
+                   : (const void*)scatter_fast_kernel<D, unsigned long long, true>);
+      if (isz == 4) scatter_fast_kernel<D, unsigned, true><<<(unsigned)fb, pthreads, (size_t)bytes, s>>>(a, sgn);
+      else scatter_fast_kernel<D, unsigned long long, true><<<(unsigned)fb, pthreads, (size_t)bytes, s>>>(a, sgn);
     } else {
       fb = std::min(fb, (long long)sms * 8);
       if (isz == 4) scatter_fast_kernel<D, unsigned, false><<<(unsigned)fb, THREADS, 0, s>>>(a, sgn);
@@ -281,7 +319,8 @@ void launch(ScatterArgs& a, cudaStream_t s) {
     }
   } else if (smem) {
     blocks = std::min(blocks, priv_ctas);
-    scatter_add_kernel<D, true><<<(unsigned)blocks, THREADS, (size_t)bytes, s>>>(a);
+    big((const void*)scatter_add_kernel<D, true>);
+    scatter_add_kernel<D, true><<<(unsigned)blocks, pthreads, (size_t)bytes, s>>>(a);
   } else {
     blocks = std::min(blocks, (long long)sms * 8);
     scatter_add_kernel<D, false><<<(unsigned)blocks, THREADS, 0, s>>>(a);
