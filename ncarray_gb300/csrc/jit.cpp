@@ -2254,6 +2254,18 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
     }
     const int64_t target = (int64_t)sms * tps;
     int64_t S = std::max<int64_t>(1, std::min<int64_t>(cdiv(target, nset * 256), RN / (8 * R)));
+    if (out && tape.compute_dtype == NCA_FLOAT64) {
+      // stored float64 expressions are bound by their arithmetic, so an SM with
+      // one CTA more than the others sets the time: among up to twice the
+      // splits, the best fill of the last round of CTAs over the SMs, at 4.5 % a
+      // split for its merge ((256, 100, 200) 72 -> 64 us, (256, 256, 256) 209
+      // -> 177; (128, 128, 128) keeps 3)
+      auto cost = [&](int64_t k) { return (double)(cdiv(nset * k, sms) * sms) / (double)(nset * k) * (1.0 + 0.045 * (double)k); };
+      int64_t best = S;
+      for (int64_t k = S; k <= std::min<int64_t>(2 * S + 2, std::max<int64_t>(1, RN / (8 * R))); ++k)
+        if (cost(k) < cost(best)) best = k;
+      S = best;
+    }
     int64_t C = cdiv(RN, S);
     S = cdiv(RN, C);
     const WordLayout L = word_layout(sp.nops, sp.nd, sp.nscal, sp.nred, sp.ptrmask != 0);
@@ -2426,7 +2438,11 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
   // outer-axis benchmarks and C1: max over axis 1 0.77 -> 0.81 of measured);
   // splits for 1024 threads per SM, 512 for short reduced axes (the tuner's
   // choices: (4096, 16384) over axis 0 and C1's 128 rows)
-  if (rows_ok && !k4r_off()) run_k4(108, k4r_persistent() ? 0 : (RN <= 256 ? 512 : 1024), k4r_lastcta());
+  // (stored float64 expressions take 2 rows at a time: 8 copies of a tape with
+  // its integer-pipe square root leave the instruction cache, (256, 256, 256)
+  // a*b + sqrt|c| - a/2 252 us against 209)
+  if (rows_ok && !k4r_off())
+    run_k4(out && tape.compute_dtype == NCA_FLOAT64 ? 102 : 108, k4r_persistent() ? 0 : (RN <= 256 ? 512 : 1024), k4r_lastcta());
   else run_k4(4, 1024, 0);
   return true;
 }
