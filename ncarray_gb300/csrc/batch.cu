@@ -364,7 +364,7 @@ __global__ void batch_persistent_kernel(const ItemDev* __restrict__ items, const
     const unsigned want = (unsigned)it.nchunks * (unsigned)NW;
     unsigned prev = 0;
     if (lane == 0) {
-      parts[c * NW + wid] = p;
+      parts[(long long)(it.first_chunk + ch.index) * NW + wid] = p;
       __threadfence();
       prev = atomicAdd(done + ch.item, 1u);
     }
@@ -502,6 +502,11 @@ void build_chunks(nca_batch* B, cudaStream_t s) {
     items[i].pad = 0;
   }
   B->nchunks = (long long)chunks.size();
+  // largest chunks first: CTA g walks chunks g, g + grid, ..., so what the CTAs
+  // move differs by at most one chunk. In array order the short chunks (ends
+  // of arrays, short arrays) fell on the CTAs at random (2000 arrays of 64 .. 4
+  // Mi elements, 256 KiB chunks: 542 -> 514 us)
+  nca::order_chunks(chunks, [](const ChunkDev& c) { return (long long)(c.e - c.a); });
   using nca::check_cuda;
   if (!B->d_items) check_cuda(cudaMalloc(&B->d_items, sizeof(ItemDev) * std::max(B->n, 1)), "batch items");
   if (!B->d_done) {
@@ -588,6 +593,9 @@ int32_t nca_batch_create(const nca_batch_item* items, int32_t n_items, nca_batch
       B->dev = current_device();
       B->items.assign(items, items + n_items);
       B->shape_class = shape_class(B);
+      long long total = 0;
+      for (const auto& it : B->items) total += it.length * (it.dtype == NCA_FLOAT32 ? 4 : 2);
+      B->chunk_bytes = chunk_bytes_for(total, (long long)sm_count(B->dev) * B->ctas_per_sm, B->slab);
       load_tuned(B);
       // NCA_BATCH_SCHEDULE="<chunk bytes>,<threads>,<slab bytes>,<CTAs per SM>" overrides the tuned schedule
       if (const char* e = getenv("NCA_BATCH_SCHEDULE")) {

@@ -54,7 +54,7 @@ struct ItemDev {            // NcaBItem in the generated source
 
 struct ChunkDev {           // NcaBChunk
   int item;
-  int pad;
+  int index;                // chunk number within the item
   long long begin;
   long long count;
 };
@@ -94,7 +94,7 @@ int op_kind(int op) {   // 0 sum (sum, mean), 1 max (max, argmax), 2 min (min, a
 // Static part of the generated source: tables, loads, accumulators, block merge.
 const char* kBatchCommon = R"NCB(
 struct NcaBItem { const void* data; long long length; int prog; int first_chunk; int nchunks; int pad; };
-struct NcaBChunk { int item; int pad; long long begin; long long count; };
+struct NcaBChunk { int item; int index; long long begin; long long count; };
 struct NcaBPart { double s; double v; long long i; long long pad; };
 struct NcaBRes { double value; long long index; };
 struct NcaBArgs {
@@ -595,7 +595,7 @@ struct nca_batch_expr {
   void* d_cnt = nullptr;
   void* d_scal = nullptr;
   long long nchunks = 0;
-  long long chunk_bytes = 512 * 1024;   // fastest with 4 loads in flight and 4 CTAs per SM on 20,000 uneven arrays
+  long long chunk_bytes = 512 * 1024;
   int unroll = 4;          // 16-byte loads per thread issued together in the walkers
   int ctas_per_sm = 4;
   bool pipe = true;        // a producer warp streams the chunks through shared-memory slabs
@@ -693,7 +693,8 @@ std::string gen_batch_source(const nca_batch_expr& b) {
         os << "      if (it.nchunks == 1) nca_bstore(A.res + (long long)c.item * " << NCA_BATCH_MAX_OUTS << " + " << o
            << ", " << pg.op[o] << ", m, it.length, " << none << ");\n";
       }
-      os << "      if (it.nchunks > 1) A.parts[cid * " << NCA_BATCH_MAX_OUTS << " + " << a << "] = m;\n    }\n  }\n";
+      os << "      if (it.nchunks > 1) A.parts[(long long)(it.first_chunk + c.index) * " << NCA_BATCH_MAX_OUTS << " + " << a
+         << "] = m;\n    }\n  }\n";
     }
     os << "}\n";
     // the merge of an item's partials (chunk order), then its final values
@@ -796,14 +797,18 @@ extern "C" int32_t nca_batch_expr_create(const nca_batch_expr_item* items, int32
     std::map<Program, int> prog_id;
     std::vector<ItemDev> hi((size_t)n_items);
     std::vector<ChunkDev> hc;
+    long long total = 0;
+    for (int i = 0; i < n_items; ++i)
+      if (items[i].length > 0 && dtype_valid(items[i].dtype)) total += items[i].length * dtinfo(items[i].dtype).size;
     // schedule knobs: chunk bytes, 16-byte loads per thread in flight, CTAs per SM
-    if (const char* e = getenv("NCA_BATCH_EXPR_CHUNK")) b->chunk_bytes = std::max(4096ll, atoll(e));
     if (const char* e = getenv("NCA_BATCH_EXPR_UNROLL")) b->unroll = std::max(1, std::min(16, atoi(e)));
     if (const char* e = getenv("NCA_BATCH_EXPR_CTAS")) b->ctas_per_sm = std::max(1, std::min(8, atoi(e)));
     if (const char* e = getenv("NCA_BATCH_EXPR_PIPE")) b->pipe = e[0] != '0';
     if (const char* e = getenv("NCA_BATCH_EXPR_SLAB")) b->slab = std::max(1024, std::min(65536, atoi(e) / 16 * 16));
     if (const char* e = getenv("NCA_BATCH_EXPR_NSLAB")) b->nslab = std::max(2, std::min(8, atoi(e)));
     if (b->pipe && !getenv("NCA_BATCH_EXPR_CTAS")) b->ctas_per_sm = 3;
+    b->chunk_bytes = chunk_bytes_for(total, (long long)sm_count(b->dev) * b->ctas_per_sm, b->slab);
+    if (const char* e = getenv("NCA_BATCH_EXPR_CHUNK")) b->chunk_bytes = std::max(4096ll, atoll(e));
     for (int i = 0; i < n_items; ++i) {
       const nca_batch_expr_item& it = items[i];
       if (it.length < 0) fail(NCA_ERR_SHAPE, "item %d: negative length", i);
@@ -836,11 +841,13 @@ extern "C" int32_t nca_batch_expr_create(const nca_batch_expr_item* items, int32
       hi[(size_t)i] = ItemDev{it.data, it.length, pid, (int)hc.size(), (int)nc, (int)isz};
       for (long long c = 0; c < nc; ++c) {
         const long long beg = c * per;
-        hc.push_back(ChunkDev{i, 0, beg, std::min(per, it.length - beg)});
+        hc.push_back(ChunkDev{i, (int)c, beg, std::min(per, it.length - beg)});
       }
       if (hc.size() > (size_t)0x7fffffff) fail(NCA_ERR_LIMIT, "too many chunks");
     }
     b->nchunks = (long long)hc.size();
+    // largest chunks first (as in batch.cu): the CTAs' shares differ by one chunk at most
+    order_chunks(hc, [&](const ChunkDev& c) { return c.count * (long long)hi[(size_t)c.item].pad; });
     cudaStream_t s = (cudaStream_t)stream;
     auto upload = [&](void** dst, const void* src, size_t bytes) {
       check_cuda(cudaMalloc(dst, std::max<size_t>(bytes, 16)), "cudaMalloc(batch tables)");

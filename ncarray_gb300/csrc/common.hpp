@@ -6,10 +6,12 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <vector>
 
 #include "../../include/ncgb300.h"
 
@@ -104,5 +106,31 @@ struct StreamScratch {
   StreamScratch(const StreamScratch&) = delete;
   StreamScratch& operator=(const StreamScratch&) = delete;
 };
+
+// ---- chunk tables of the batched kernels --------------------------------------
+// Bytes per chunk: about 4 chunks for each of `ctas` CTAs, in whole slabs,
+// between 64 and 512 KiB. Larger chunks have fewer ends (trees, counts) and
+// leave more of the last round idle: 2000 arrays, 2.2 GB, at 128 / 256 / 384 /
+// 512 / 1024 KiB 597 / 551 / 530 / 525 / 530 us; 600 arrays through the general
+// form, 0.66 GB, at 64 / 128 / 256 / 384 KiB 254 / 216 / 201 / 197 us.
+inline long long chunk_bytes_for(long long total, long long ctas, long long slab) {
+  const long long want = total / (ctas * 4) / slab * slab;
+  return std::min<long long>(512 * 1024, std::max<long long>(64 * 1024, want));
+}
+// Stable order by descending size, in linear time: 64 classes per power of two.
+template <class C, class F>
+void order_chunks(std::vector<C>& chunks, F bytes) {
+  auto cls = [&](const C& c) {
+    const unsigned long long b = (unsigned long long)std::max<long long>(bytes(c), 0) + 64;
+    int lg = 63 - __builtin_clzll(b);
+    return lg * 64 + (int)((b >> (lg - 6)) & 63);
+  };
+  std::vector<int> start(64 * 64 + 1, 0);
+  for (const C& c : chunks) ++start[(size_t)(64 * 64 - 1 - cls(c)) + 1];
+  for (size_t k = 1; k < start.size(); ++k) start[k] += start[k - 1];
+  std::vector<C> out(chunks.size());
+  for (const C& c : chunks) out[(size_t)start[(size_t)(64 * 64 - 1 - cls(c))]++] = c;
+  chunks.swap(out);
+}
 
 }  // namespace nca
