@@ -6,6 +6,7 @@ API without it raises: there is no CPU fallback on the device path.
 from __future__ import annotations
 
 import ctypes
+import struct
 from ctypes import POINTER, c_char_p, c_double, c_float, c_int32, c_int64, c_uint32, c_uint64, c_void_p
 from pathlib import Path
 
@@ -148,23 +149,24 @@ def check(status: int) -> None:
 
 
 def call(name: str, *args) -> None:
-    check(getattr(lib(), name)(*args))
+    status = getattr(_lib or lib(), name)(*args)
+    if status != OK:
+        check(status)
 
 
 VIEW_SUBOFFSETS = 1   # nca_view.flags: PEP 3118 suboffset semantics on the pointer axis
 
 
+_VIEW = struct.Struct("=Qii%dq%dq%dqii" % (MAX_NDIM, MAX_NDIM, MAX_NDIM))   # the fields of View, which has no padding
+assert _VIEW.size == ctypes.sizeof(View)
+_PAD = tuple((0,) * (MAX_NDIM - n) for n in range(MAX_NDIM + 1))
+_NO_OFFSETS = (0,) * MAX_NDIM
+
+
 def make_view(ptr: int, dtype: int, shape, byte_strides, byte_offset: int = 0) -> View:
-    v = View()
-    v.data = ptr + byte_offset if ptr else None
-    v.dtype = int(dtype)
-    v.ndim = len(shape)
-    if v.ndim > MAX_NDIM:
+    n = len(shape)
+    if n > MAX_NDIM:
         raise ValueError(f"at most {MAX_NDIM} dims")
-    for d, (n, s) in enumerate(zip(shape, byte_strides)):
-        v.shape[d] = int(n)
-        v.strides[d] = int(s)
-        v.offsets[d] = 0
-    v.pointer_axis = -1
-    v.flags = 0
-    return v
+    pad = _PAD[n]
+    return View.from_buffer_copy(_VIEW.pack(ptr + byte_offset if ptr else 0, int(dtype), n, *map(int, shape), *pad,
+                                            *map(int, byte_strides), *pad, *_NO_OFFSETS, -1, 0))

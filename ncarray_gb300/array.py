@@ -39,21 +39,42 @@ def lazy_mode():
         _EAGER[0] = old
 
 
+_TORCH = None
+_RAW_STREAM = None   # torch's current raw stream of a device, once CUDA is initialised
+
+
 def _torch():
-    import torch
-    return torch
+    global _TORCH
+    if _TORCH is None:
+        import torch
+        _TORCH = torch
+    return _TORCH
 
 
 def current_stream() -> int:
+    global _RAW_STREAM
     torch = _torch()
-    return int(torch.cuda.current_stream().cuda_stream)
+    if _RAW_STREAM is None:
+        stream = int(torch.cuda.current_stream().cuda_stream)   # initialises CUDA
+        get, dev = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+        if get is not None and dev is not None:
+            _RAW_STREAM = lambda: get(dev())  # noqa: E731
+        return stream
+    return _RAW_STREAM()
+
+
+_DEVICES: dict = {}   # torch devices by index, once CUDA is known to be there
 
 
 def _device():
     torch = _torch()
-    if not torch.cuda.is_available():
+    if not _DEVICES and not torch.cuda.is_available():
         raise RuntimeError("ncarray_gb300 device arrays need a CUDA device")
-    return torch.device("cuda", torch.cuda.current_device())
+    i = torch.cuda.current_device()
+    d = _DEVICES.get(i)
+    if d is None:
+        d = _DEVICES[i] = torch.device("cuda", i)
+    return d
 
 
 def _c_strides(shape: Sequence[int], itemsize: int) -> list[int]:
@@ -69,15 +90,15 @@ class NCDevArray:
 
     def __init__(self, shape: Sequence[int] = (), dtype: DType = DType.float64, *, _buf=None,
                  _offset: int = 0, _strides: Optional[Sequence[int]] = None):
-        self.dtype = DType(dtype)
-        self.shape = tuple(int(n) for n in shape)
+        self.dtype = dtype if type(dtype) is DType else DType(dtype)
+        self.shape = tuple(map(int, shape))
         isz = ITEMSIZE[self.dtype]
         if _buf is None:
-            nbytes = max(self.size * isz, 1)
-            _buf = _torch().empty(nbytes, dtype=_torch().uint8, device=_device())
+            torch = _torch()
+            _buf = torch.empty(max(self.size * isz, 1), dtype=torch.uint8, device=_device())
         self._buf = _buf
         self._offset = int(_offset)
-        self.strides = tuple(int(s) for s in (_strides if _strides is not None else _c_strides(self.shape, isz)))
+        self.strides = tuple(map(int, _strides if _strides is not None else _c_strides(self.shape, isz)))
         # pointer-axis views (from_panels): axis 0 indexes a device table of
         # panel pointers; None for ordinary arrays
         self._ptr = None
@@ -412,6 +433,9 @@ def _as_node(x):
     return DevExpr.const(x)
 
 
+_LOAD, _LOAD_SO, _CONST = int(OpCode.LOAD_NCARR), int(OpCode.LOAD_SOARR), int(OpCode.LOAD_CONST)
+
+
 class DevExpr:
     """A lazy tape (RPN instructions over array operands and scalars)."""
 
@@ -427,7 +451,7 @@ class DevExpr:
     def leaf(cls, a: NCDevArray) -> "DevExpr":
         e = cls()
         e.arrays.append(a)
-        e.instrs.append((OpCode.LOAD_NCARR << 24) | 0)
+        e.instrs.append(_LOAD << 24)
         e.work = e.expr_dtype = a.dtype
         return e
 
@@ -436,7 +460,7 @@ class DevExpr:
         e = cls()
         dt = scalar_dtype(v)
         e.scalars.append((dt, scalar_slot(v, dt)))
-        e.instrs.append((OpCode.LOAD_CONST << 24) | 0)
+        e.instrs.append(_CONST << 24)
         e.work = e.expr_dtype = dt
         return e
 
@@ -453,21 +477,22 @@ class DevExpr:
     def _append(self, other: "DevExpr") -> None:
         # an operand view that is already on the tape is loaded through the same
         # index (one load per element instead of two)
-        keys = {_view_key(a): i for i, a in enumerate(self.arrays)}
         remap = []
-        for a in other.arrays:
-            k = _view_key(a)
-            if k not in keys:
-                keys[k] = len(self.arrays)
-                self.arrays.append(a)
-            remap.append(keys[k])
+        if other.arrays:
+            keys = {_view_key(a): i for i, a in enumerate(self.arrays)} if self.arrays else {}
+            for a in other.arrays:
+                k = _view_key(a)
+                if k not in keys:
+                    keys[k] = len(self.arrays)
+                    self.arrays.append(a)
+                remap.append(keys[k])
         ns = len(self.scalars)
         self.scalars += other.scalars
         for ins in other.instrs:
             op, idx = ins >> 24, ins & 0xFFFFFF
-            if op in (OpCode.LOAD_NCARR, OpCode.LOAD_SOARR):
+            if op == _LOAD or op == _LOAD_SO:
                 ins = (op << 24) | remap[idx]
-            elif op == OpCode.LOAD_CONST:
+            elif op == _CONST:
                 ins = (op << 24) | (idx + ns)
             self.instrs.append(ins)
         if getattr(other, "_iota_shape", None) is not None and getattr(self, "_iota_shape", None) is None:
@@ -489,13 +514,13 @@ class DevExpr:
         e._append(b)
         e.work = promote(a.work, b.work)
         e.expr_dtype = result_dtype(op, e.work)
-        e.instrs.append(op << 24)
+        e.instrs.append(int(op) << 24)
         return e._finish()
 
     def _unary(self, op: OpCode):
         e = self._clone()
         e.expr_dtype = result_dtype(op, e.work)
-        e.instrs.append(op << 24)
+        e.instrs.append(int(op) << 24)
         return e._finish()
 
     def _finish(self):
@@ -511,6 +536,8 @@ class DevExpr:
         shapes = [a.shape for a in self.arrays]
         if getattr(self, "_iota_shape", None) is not None:
             shapes.append(self._iota_shape)
+        if shapes and all(s == shapes[0] for s in shapes):
+            return tuple(shapes[0])
         n = max((len(s) for s in shapes), default=0)
         out = [1] * n
         for s in shapes:
@@ -526,14 +553,8 @@ class DevExpr:
         ins = (ctypes.c_uint32 * max(len(self.instrs), 1))(*self.instrs)
         sd = (ctypes.c_int32 * max(len(self.scalars), 1))(*[int(d) for d, _ in self.scalars])
         ss = (ctypes.c_uint64 * max(len(self.scalars), 1))(*[s for _, s in self.scalars])
-        t = _lib.Tape()
-        t.instrs = ctypes.cast(ins, ctypes.POINTER(ctypes.c_uint32))
-        t.n_instrs = len(self.instrs)
-        t.n_scalars = len(self.scalars)
-        t.scalar_dtypes = ctypes.cast(sd, ctypes.POINTER(ctypes.c_int32))
-        t.scalar_slots = ctypes.cast(ss, ctypes.POINTER(ctypes.c_uint64))
-        t.compute_dtype = int(compute_dtype(self.expr_dtype, self.work))
-        t.result_dtype = int(self.expr_dtype)
+        t = _lib.Tape(ins, len(self.instrs), len(self.scalars), sd, ss, int(compute_dtype(self.expr_dtype, self.work)),
+                      int(self.expr_dtype))
         return t, (ins, sd, ss)
 
     def _operands(self):
@@ -572,11 +593,10 @@ class DevExpr:
             return []
         shape = out.shape if out is not None else self.shape
         results, rarr = _reductions(shape, self.expr_dtype, reductions, red_out)
-        rs = list(rarr)
         if out is not None and out.size == 0:
             out = None
         _lib.call("nca_expr_reduce", ctypes.byref(t), ops, n,
-                  ctypes.byref(out.view_struct()) if out is not None else None, rarr, len(rs), stream)
+                  ctypes.byref(out.view_struct()) if out is not None else None, rarr, len(results), stream)
         return results
 
     # ---- host <-> device copies of views (nca_copy_host) ----
@@ -644,26 +664,31 @@ class DevExpr:
 def _reductions(shape, expr_dtype: DType, reductions, red_out):
     """The result arrays of (RedOp, axes) reductions of a value of `shape` and
     their C descriptors (one shared axes mask)."""
-    results, rs = [], []
+    results = []
+    reductions = list(reductions)
+    rs = (_lib.Reduction * max(len(reductions), 1))()
+    first = None
     for i, (op, axes) in enumerate(reductions):
-        op = RedOp(op)
+        op = op if type(op) is RedOp else RedOp(op)
         mask, kept = _axes_mask(axes, len(shape))
         odt = _red_out_dtype(op, expr_dtype)
+        want = tuple([shape[d] for d in kept])
         if red_out is not None:
             res = red_out[i]
-            if res.dtype != odt or res.shape != tuple(shape[d] for d in kept):
+            if res.dtype != odt or res.shape != want:
                 raise ValueError(f"reduction output {i} must be {odt.name} {[shape[d] for d in kept]}")
         else:
-            res = NCDevArray([shape[d] for d in kept], odt)
+            res = NCDevArray(want, odt)
         results.append(res)
-        r = _lib.Reduction()
+        r = rs[i]
         r.op = int(op)
         r.axes_mask = mask
         r.out = res.view_struct()
-        rs.append(r)
-    if len({r.axes_mask for r in rs}) > 1:
-        raise ValueError("one evaluate() call reduces over one set of axes")
-    return results, (_lib.Reduction * max(len(rs), 1))(*rs)
+        if first is None:
+            first = mask
+        elif mask != first:
+            raise ValueError("one evaluate() call reduces over one set of axes")
+    return results, rs
 
 
 def evaluate_many(outputs, reductions: Iterable = (), red_out=None):
@@ -703,20 +728,19 @@ def evaluate_many(outputs, reductions: Iterable = (), red_out=None):
                         if (ins >> 24) in (OpCode.LOAD_NCARR, OpCode.LOAD_SOARR) else ins for ins in e.instrs]
             e = r
         tapes.append(e._tape())
-    reductions = list(reductions)
     results, rarr = _reductions(shape, exprs[0].expr_dtype, reductions, red_out)
     tarr = (_lib.Tape * len(tapes))(*[t for t, _ in tapes])
     ops = (_lib.View * max(len(arrays), 1))(*[a.view_struct() for a in arrays])
     oarr = (_lib.View * len(outs))(*[o.view_struct() for o in outs])
     if all(o.size for o in outs):
-        _lib.call("nca_expr_multi", tarr, len(tapes), ops, len(arrays), oarr, rarr, len(reductions), current_stream())
+        _lib.call("nca_expr_multi", tarr, len(tapes), ops, len(arrays), oarr, rarr, len(results), current_stream())
     return results
 
 
 def _view_key(a: NCDevArray):
-    if a._ptr is not None:
-        return (a.ptr, int(a.dtype), a.shape, a.strides, "ptr", a._ptr["poff"], a._ptr["step"])
-    return (a.ptr, int(a.dtype), a.shape, a.strides)
+    if a._ptr is None:
+        return (a.ptr, a.dtype, a.shape, a.strides)
+    return (a.ptr, a.dtype, a.shape, a.strides, "ptr", a._ptr["poff"], a._ptr["step"])
 
 
 def _axes_mask(axes, ndim: int):

@@ -10,6 +10,9 @@ Type rules restated from:
 from __future__ import annotations
 
 import enum
+import functools
+import math
+import struct
 
 import numpy as np
 
@@ -106,17 +109,20 @@ def from_numpy(npdt) -> DType:
     raise TypeError(f"numpy dtype {npdt} has no ncarray counterpart")
 
 
+@functools.lru_cache(maxsize=None)
 def arith(dt: DType) -> DType:
     """float32 stands in for the 16-bit float storage types in arithmetic."""
     return DType.float32 if dt in (DType.bfloat16, DType.float16) else DType(dt)
 
 
+@functools.lru_cache(maxsize=None)
 def promote(a: DType, b: DType) -> DType:
     """promote_expr_types: the numerically larger DType."""
     a, b = arith(a), arith(b)
     return a if int(a) >= int(b) else b
 
 
+@functools.lru_cache(maxsize=None)
 def sum_type(dt: DType) -> DType:
     dt = DType(dt)
     if dt in (DType.bool, DType.uint8, DType.uint16):
@@ -126,6 +132,7 @@ def sum_type(dt: DType) -> DType:
     return arith(dt)
 
 
+@functools.lru_cache(maxsize=None)
 def diff_type(dt: DType) -> DType:
     dt = DType(dt)
     if dt in (DType.bool, DType.uint8, DType.uint16, DType.int8, DType.int16):
@@ -133,6 +140,7 @@ def diff_type(dt: DType) -> DType:
     return arith(dt)
 
 
+@functools.lru_cache(maxsize=None)
 def result_dtype(op: OpCode, work: DType) -> DType:
     """determine_dtype_for_op(op, work)."""
     work = arith(work)
@@ -150,6 +158,7 @@ def result_dtype(op: OpCode, work: DType) -> DType:
     return work
 
 
+@functools.lru_cache(maxsize=None)
 def compute_dtype(expr_dt: DType, work: DType) -> DType:
     """The VM's WorkT: the result dtype, or the work dtype for bool results."""
     return arith(work) if expr_dt == DType.bool else arith(expr_dt)
@@ -175,8 +184,26 @@ def scalar_dtype(value) -> DType:
     raise TypeError(f"unsupported scalar {value!r}")
 
 
+# Python ints of these ranges are carried as their two's complement bytes; an
+# int outside its type's range is left to numpy's conversion
+_INT_RANGE = {t: (-(1 << (b - 1)), (1 << (b - 1)) - 1, (1 << b) - 1) if signed else (0, (1 << b) - 1, (1 << b) - 1)
+              for t, b, signed in ((DType.uint8, 8, False), (DType.uint16, 16, False), (DType.uint32, 32, False),
+                                   (DType.uint64, 64, False), (DType.int8, 8, True), (DType.int16, 16, True),
+                                   (DType.int32, 32, True), (DType.int64, 64, True))}
+
+
 def scalar_slot(value, dt: DType) -> int:
     """8-byte slot carrying `value` as dtype `dt`."""
+    t = type(value)
+    if t is int and dt in _INT_RANGE:
+        lo, hi, mask = _INT_RANGE[dt]
+        if lo <= value <= hi:
+            return value & mask
+    if t is float and math.isfinite(value) and abs(value) < 3e38:
+        if dt == DType.float32:
+            return int.from_bytes(struct.pack("<f", value), "little")
+        if dt == DType.float64:
+            return int.from_bytes(struct.pack("<d", value), "little")
     dt = DType(dt)
     if dt == DType.bfloat16:
         b = np.array([value], dtype=np.float32).view(np.uint32)[0] >> 16
