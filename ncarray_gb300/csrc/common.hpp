@@ -107,6 +107,10 @@ struct StreamScratch {
   StreamScratch& operator=(const StreamScratch&) = delete;
 };
 
+// `n` arrival counters, all zero, for a kernel on stream `s` that leaves them
+// zero; null where the caller has to zero counters of its own.
+uint32_t* arrival_counters(int64_t n, cudaStream_t s);
+
 // ---- chunk tables of the batched kernels --------------------------------------
 // Bytes per chunk: about 4 chunks for each of `ctas` CTAs, in whole slabs,
 // between 64 and 512 KiB. Larger chunks have fewer ends (trees, counts) and

@@ -2134,21 +2134,19 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
       }
       // block teams over few kept positions (global reductions): the CTA that
       // stores the last partial of a kept position merges them in the order the
-      // finalize pass uses (one arrival counter per kept position, zeroed here),
-      // so there is no second launch and the result is the same
+      // finalize pass uses (one arrival counter per kept position), so there is no second launch and the result is the same
       sp.lastcta = (S > 1 && sp.team == 256 && KN <= 64) ? 1 : 0;
       const size_t pbytes = S > 1 ? (size_t)(S * KN) * 8 * ((has_sum ? 1 : 0) + (has_max ? 2 : 0) + (has_min ? 2 : 0)) : 0;
-      const size_t cbytes = sp.lastcta ? ((size_t)KN * 4 + 255) / 256 * 256 : 0;
+      uint32_t* cnt = sp.lastcta ? arrival_counters(KN, stream) : nullptr;
+      const size_t cbytes = sp.lastcta && !cnt ? ((size_t)KN * 4 + 255) / 256 * 256 : 0;
       StreamScratch part(pbytes + cbytes, stream);
       if (S > 1) {
         uint64_t* p = (uint64_t*)part.ptr;
         if (has_sum) { w[L.psum] = (uint64_t)(uintptr_t)p; p += S * KN; }
         if (has_max) { w[L.pmax] = (uint64_t)(uintptr_t)p; p += 2 * S * KN; }
         if (has_min) { w[L.pmin] = (uint64_t)(uintptr_t)p; p += 2 * S * KN; }
-        if (sp.lastcta) {
-          w[L.aux] = (uint64_t)(uintptr_t)p;
-          check_cuda(cudaMemsetAsync(p, 0, cbytes, stream), "arrival counters");
-        }
+        w[L.aux] = (uint64_t)(uintptr_t)(cnt ? (void*)cnt : (void*)p);
+        if (cbytes) check_cuda(cudaMemsetAsync(p, 0, cbytes, stream), "arrival counters");
       }
       CUfunction fn = kernel_for(sp, tape);
       // warp and smaller teams stride over their units from a few blocks per SM
@@ -2238,14 +2236,15 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
       w[L.nsplit] = (uint64_t)G; w[L.chunk] = 0; w[L.keptn] = (uint64_t)KN; w[L.redn] = (uint64_t)RN;
       const int64_t slots = (G + nset) * GPC * sp.vec;
       const size_t pbytes = (size_t)slots * 8 * ((has_sum ? 1 : 0) + (has_max ? 2 : 0) + (has_min ? 2 : 0));
-      const size_t cbytes = ((size_t)nset * 4 + 255) / 256 * 256;
+      uint32_t* cnt = arrival_counters(nset, stream);
+      const size_t cbytes = cnt ? 0 : ((size_t)nset * 4 + 255) / 256 * 256;
       StreamScratch part(pbytes + cbytes, stream);
       uint64_t* p = (uint64_t*)part.ptr;
       if (has_sum) { w[L.psum] = (uint64_t)(uintptr_t)p; p += slots; }
       if (has_max) { w[L.pmax] = (uint64_t)(uintptr_t)p; p += 2 * slots; }
       if (has_min) { w[L.pmin] = (uint64_t)(uintptr_t)p; p += 2 * slots; }
-      w[L.aux] = (uint64_t)(uintptr_t)p;
-      check_cuda(cudaMemsetAsync(p, 0, cbytes, stream), "arrival counters");
+      w[L.aux] = (uint64_t)(uintptr_t)(cnt ? (void*)cnt : (void*)p);
+      if (cbytes) check_cuda(cudaMemsetAsync(p, 0, cbytes, stream), "arrival counters");
       launch(fn, G, w, stream);
       sp.k4r = 0;
       sp.rd = 0;
@@ -2274,17 +2273,16 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
     w[L.nsplit] = (uint64_t)S; w[L.chunk] = (uint64_t)C; w[L.keptn] = (uint64_t)KN; w[L.redn] = (uint64_t)RN;
     sp.lastcta = (lastcta && S > 1) ? 1 : 0;
     const size_t pbytes = S > 1 ? (size_t)(S * KN) * 8 * ((has_sum ? 1 : 0) + (has_max ? 2 : 0) + (has_min ? 2 : 0)) : 0;
-    const size_t cbytes = sp.lastcta ? ((size_t)nset * 4 + 255) / 256 * 256 : 0;
+    uint32_t* cnt = sp.lastcta ? arrival_counters(nset, stream) : nullptr;
+    const size_t cbytes = sp.lastcta && !cnt ? ((size_t)nset * 4 + 255) / 256 * 256 : 0;
     StreamScratch part(pbytes + cbytes, stream);
     if (S > 1) {
       uint64_t* p = (uint64_t*)part.ptr;
       if (has_sum) { w[L.psum] = (uint64_t)(uintptr_t)p; p += S * KN; }
       if (has_max) { w[L.pmax] = (uint64_t)(uintptr_t)p; p += 2 * S * KN; }
       if (has_min) { w[L.pmin] = (uint64_t)(uintptr_t)p; p += 2 * S * KN; }
-      if (sp.lastcta) {
-        w[L.aux] = (uint64_t)(uintptr_t)p;
-        check_cuda(cudaMemsetAsync(p, 0, cbytes, stream), "arrival counters");
-      }
+      w[L.aux] = (uint64_t)(uintptr_t)(cnt ? (void*)cnt : (void*)p);
+      if (cbytes) check_cuda(cudaMemsetAsync(p, 0, cbytes, stream), "arrival counters");
     }
     CUfunction fn = kernel_for(sp, tape);
     launch(fn, nset * S, w, stream);
@@ -2309,20 +2307,19 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
     w[L.nsplit] = (uint64_t)S; w[L.chunk] = (uint64_t)C; w[L.keptn] = (uint64_t)KN; w[L.redn] = (uint64_t)RN;
     // lastcta: when the kept groups fill whole 256-thread blocks, the last of
     // the S blocks over a set of kept groups merges their partials (one arrival
-    // counter per set, zeroed here) instead of a finalize launch; a tuned choice
+    // counter per set) instead of a finalize launch; a tuned choice
     sp.lastcta = (lastcta && S > 1 && KG % 256 == 0) ? 1 : 0;
     const size_t pbytes = S > 1 ? (size_t)(S * KN) * 8 * ((has_sum ? 1 : 0) + (has_max ? 2 : 0) + (has_min ? 2 : 0)) : 0;
-    const size_t cbytes = sp.lastcta ? ((size_t)(KG / 256) * 4 + 255) / 256 * 256 : 0;
+    uint32_t* cnt = sp.lastcta ? arrival_counters(KG / 256, stream) : nullptr;
+    const size_t cbytes = sp.lastcta && !cnt ? ((size_t)(KG / 256) * 4 + 255) / 256 * 256 : 0;
     StreamScratch part(pbytes + cbytes, stream);
     if (S > 1) {
       uint64_t* p = (uint64_t*)part.ptr;
       if (has_sum) { w[L.psum] = (uint64_t)(uintptr_t)p; p += S * KN; }
       if (has_max) { w[L.pmax] = (uint64_t)(uintptr_t)p; p += 2 * S * KN; }
       if (has_min) { w[L.pmin] = (uint64_t)(uintptr_t)p; p += 2 * S * KN; }
-      if (sp.lastcta) {
-        w[L.aux] = (uint64_t)(uintptr_t)p;
-        check_cuda(cudaMemsetAsync(p, 0, cbytes, stream), "arrival counters");
-      }
+      w[L.aux] = (uint64_t)(uintptr_t)(cnt ? (void*)cnt : (void*)p);
+      if (cbytes) check_cuda(cudaMemsetAsync(p, 0, cbytes, stream), "arrival counters");
     }
     CUfunction fn = kernel_for(sp, tape);
     launch(fn, cdiv(KG * S, 256), w, stream);

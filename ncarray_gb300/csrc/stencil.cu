@@ -21,6 +21,7 @@
 #include <cstring>
 
 #include <mutex>
+#include <unordered_map>
 
 #include "common.hpp"
 #include "mbar.cuh"
@@ -728,6 +729,13 @@ void run(const nca_view* a, const nca_view* b, const double* w27, double dt, int
 
 }  // namespace
 
+namespace {
+// Arrival counters of kernels whose last CTA merges the partial results, one
+// block of them per stream (see arrival_counters). Zero when the module loads.
+constexpr int ARR_STREAMS = 64, ARR_N = 16384;
+__device__ uint32_t g_arrivals[ARR_STREAMS][ARR_N];
+}  // namespace
+
 namespace nca {
 // address of the status word of JIT kernels on the current device
 int* jit_status_word() {
@@ -742,6 +750,43 @@ int* jit_status_word() {
     addr[dev] = static_cast<int*>(p);
   }
   return addr[dev];
+}
+
+// Kernels of one stream run one after the other, so a block of counters that
+// every kernel leaves zero (its last CTA resets what it used) serves all of a
+// stream's kernels without a memset before each: (4096, 16384) float32 summed
+// over axis 0 59.7 -> 54.9 us, of which the memset was 1.5 and the gaps around it the rest. Streams are told apart by
+// their id, which no later stream gets again. Null, and the caller zeroes
+// counters of its own: for a stream under capture (its graph may run on
+// several streams at once), past the first ARR_STREAMS streams of a device and
+// above ARR_N counters.
+uint32_t* arrival_counters(int64_t n, cudaStream_t stream) {
+  static std::mutex mu;
+  struct Dev { uint32_t* base = nullptr; std::unordered_map<unsigned long long, int> slot; };
+  static Dev devs[64];
+  if (n > ARR_N) return nullptr;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone ||
+      cudaStreamGetId(stream, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  const int dev = current_device();
+  if (dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lk(mu);
+  Dev& d = devs[dev];
+  if (!d.base) {
+    void* p = nullptr;
+    check_cuda(cudaGetSymbolAddress(&p, g_arrivals), "arrival counters");
+    d.base = static_cast<uint32_t*>(p);
+  }
+  auto it = d.slot.find(id);
+  if (it == d.slot.end()) {
+    if ((int)d.slot.size() >= ARR_STREAMS) return nullptr;
+    it = d.slot.emplace(id, (int)d.slot.size()).first;
+  }
+  return d.base + (size_t)it->second * ARR_N;
 }
 
 // reads and clears the stencil status word (synchronises the stream)
