@@ -108,8 +108,11 @@ struct StreamScratch {
 };
 
 // `n` arrival counters, all zero, for a kernel on stream `s` that leaves them
-// zero; null where the caller has to zero counters of its own.
+// zero; null where the caller has to zero counters of its own. The marked ones
+// are for kernels that may leave any count: launch_mark() in the high half.
 uint32_t* arrival_counters(int64_t n, cudaStream_t s);
+unsigned long long* marked_counters(int64_t n, cudaStream_t s);
+uint32_t launch_mark();
 
 // ---- chunk tables of the batched kernels --------------------------------------
 // Bytes per chunk: about 4 chunks for each of `ctas` CTAs, in whole slabs,

@@ -17,6 +17,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstring>
 
@@ -731,9 +732,10 @@ void run(const nca_view* a, const nca_view* b, const double* w27, double dt, int
 
 namespace {
 // Arrival counters of kernels whose last CTA merges the partial results, one
-// block of them per stream (see arrival_counters). Zero when the module loads.
+// block of them per stream (see stream_words). Zero when the module loads.
 constexpr int ARR_STREAMS = 64, ARR_N = 16384;
 __device__ uint32_t g_arrivals[ARR_STREAMS][ARR_N];
+__device__ unsigned long long g_marked[ARR_STREAMS][ARR_N];
 }  // namespace
 
 namespace nca {
@@ -755,14 +757,17 @@ int* jit_status_word() {
 // Kernels of one stream run one after the other, so a block of counters that
 // every kernel leaves zero (its last CTA resets what it used) serves all of a
 // stream's kernels without a memset before each: (4096, 16384) float32 summed
-// over axis 0 59.7 -> 54.9 us, of which the memset was 1.5 and the gaps around it the rest. Streams are told apart by
-// their id, which no later stream gets again. Null, and the caller zeroes
-// counters of its own: for a stream under capture (its graph may run on
-// several streams at once), past the first ARR_STREAMS streams of a device and
-// above ARR_N counters.
-uint32_t* arrival_counters(int64_t n, cudaStream_t stream) {
+// over axis 0 59.7 -> 54.9 us. Streams are told apart by their id, which no
+// later stream gets again. Null, and the caller zeroes words of its own: for a
+// stream under capture (its graph may run on several streams at once), past
+// the first ARR_STREAMS streams of a device and above ARR_N words.
+//
+// Kernels with bounded waits may stop early and leave any count behind, so
+// they take marked words instead: 64 bits, the launch's mark above the count,
+// and a word with another mark counts from zero.
+static void* stream_words(bool marked, int64_t n, cudaStream_t stream) {
   static std::mutex mu;
-  struct Dev { uint32_t* base = nullptr; std::unordered_map<unsigned long long, int> slot; };
+  struct Dev { void *plain = nullptr, *marked = nullptr; std::unordered_map<unsigned long long, int> slot; };
   static Dev devs[64];
   if (n > ARR_N) return nullptr;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
@@ -776,17 +781,29 @@ uint32_t* arrival_counters(int64_t n, cudaStream_t stream) {
   if (dev < 0 || dev >= 64) return nullptr;
   std::lock_guard<std::mutex> lk(mu);
   Dev& d = devs[dev];
-  if (!d.base) {
-    void* p = nullptr;
-    check_cuda(cudaGetSymbolAddress(&p, g_arrivals), "arrival counters");
-    d.base = static_cast<uint32_t*>(p);
+  if (!d.plain) {
+    check_cuda(cudaGetSymbolAddress(&d.marked, g_marked), "marked counters");
+    check_cuda(cudaGetSymbolAddress(&d.plain, g_arrivals), "arrival counters");
   }
   auto it = d.slot.find(id);
   if (it == d.slot.end()) {
     if ((int)d.slot.size() >= ARR_STREAMS) return nullptr;
     it = d.slot.emplace(id, (int)d.slot.size()).first;
   }
-  return d.base + (size_t)it->second * ARR_N;
+  const size_t first = (size_t)it->second * ARR_N;
+  return marked ? (void*)(static_cast<unsigned long long*>(d.marked) + first)
+                : (void*)(static_cast<uint32_t*>(d.plain) + first);
+}
+uint32_t* arrival_counters(int64_t n, cudaStream_t stream) {
+  return static_cast<uint32_t*>(stream_words(false, n, stream));
+}
+unsigned long long* marked_counters(int64_t n, cudaStream_t stream) {
+  return static_cast<unsigned long long*>(stream_words(true, n, stream));
+}
+uint32_t launch_mark() {
+  static std::atomic<uint32_t> next{1};
+  uint32_t m = next++;
+  return m ? m : next++;   // 0 is what a cleared word holds
 }
 
 // reads and clears the stencil status word (synchronises the stream)

@@ -68,6 +68,36 @@ def test_capture_beside_plain_calls(cuda):
         assert int(full.to_host()) == int(want.sum())
 
 
+def test_staged_units(cuda):
+    """Transposed 4-byte operands stored and reduced: pieces of a unit split
+    between CTAs, on several streams, repeated, and in a graph beside them."""
+    rng = np.random.default_rng(4)
+    h = rng.integers(-9, 9, (64, 64, 128, 8)).astype(np.int32)    # (p, b, r, q)
+    t = nca.NCDevArray.from_host(h).transpose(3, 1, 2, 0)
+    want = h.transpose(3, 1, 2, 0) * 3
+    with nca.lazy_mode():
+        e = t * np.int32(3)
+    red = [(RedOp.SUM, 2), (RedOp.MAX, 2)]
+    out = nca.NCDevArray(want.shape, e.dtype)
+    ref = e.evaluate(out, red)
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        e.evaluate(out, red, ref)
+    sides = []
+    for s in [torch.cuda.Stream() for _ in range(3)]:
+        with torch.cuda.stream(s):
+            o = nca.NCDevArray(want.shape, e.dtype)
+            sides += [(o, e.evaluate(o, red)) for _ in range(3)]
+    g.replay()
+    g.replay()
+    torch.cuda.synchronize()
+    for o, (sm, mx) in sides + [(out, ref)]:
+        np.testing.assert_array_equal(o.to_host(), want)
+        np.testing.assert_array_equal(sm.to_host(), want.sum(axis=2))
+        np.testing.assert_array_equal(mx.to_host(), want.max(axis=2))
+
+
 def test_more_sets_than_counters(cuda):
     # (16, 16385 * 256) has more sets of 256 columns than a stream has counters
     n = 16385 * 256
