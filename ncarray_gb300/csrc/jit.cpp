@@ -366,6 +366,7 @@ struct Spec {
   // operands that do not move along it
   int rowu = 0, loopd = -1, loopf = 1;
   uint32_t invmask = 0;
+  int k4g = 0;       // row-lane form without a stored value: 1 takes unroll rows' loads together
   int k4r = 0;       // kind 4: row lanes per warp (row-lane form, one reduced dim rd); 0: thread per column group
   int rd = 0;
   int k4p = 0;       // kind 4 row-lane form on a persistent grid (equal contiguous ranges of units)
@@ -640,7 +641,7 @@ static std::string gen_source(const Spec& sp, const Tape& t) {
      << "\n#define NCA_HAS_OUT " << (sp.has_out ? 1 : 0) << "\n#define NCA_NWORDS " << L.nwords
      << "\n#define NCA_HAS_SUM " << (sp.has_sum ? 1 : 0) << "\n#define NCA_HAS_MAX " << (sp.has_max ? 1 : 0)
      << "\n#define NCA_HAS_MIN " << (sp.has_min ? 1 : 0) << "\n#define NCA_LASTCTA " << sp.lastcta
-     << "\n#define NCA_K4R " << sp.k4r << "\n#define NCA_RD " << sp.rd << "\n#define NCA_K4P " << sp.k4p
+     << "\n#define NCA_K4G " << sp.k4g << "\n#define NCA_K4R " << sp.k4r << "\n#define NCA_RD " << sp.rd << "\n#define NCA_K4P " << sp.k4p
      << "\n#define NCA_ROWU " << sp.rowu << "\n#define NCA_LOOPD " << sp.loopd << "\n#define NCA_LOOPF " << sp.loopf
      << "\n#define NCA_INVMASK " << sp.invmask << "u\n#define NCA_OUT_ES " << (sp.has_out ? dtinfo(sp.out_dtype).size : 1)
      << "\n#define NCA_K4B " << sp.k4b << "\n#define NCA_K3RV " << sp.k3rv << "\n#define NCA_K3TU " << sp.k3tu << "\n";
@@ -1158,7 +1159,7 @@ static std::string plan_key(const Spec& sp, const Tape& t) {
   add(sp.has_sum); add(sp.has_max); add(sp.has_min); add(sp.nscal); add(sp.qd); add(sp.qx); add(sp.tp);
   add(sp.rb); add(sp.tmask); add(sp.tile_bytes); add(sp.unroll); add(sp.qxp); add(sp.minb); add(sp.grp);
   add(sp.ns); add(sp.ld); add(sp.npc); add(sp.ltp8); add(sp.pmask); add(sp.umask); add(sp.nmaps); add(sp.uumask); add(sp.ptrmask);
-  add(sp.nob); add(sp.lastcta); add(sp.block); add(sp.k4r); add(sp.rd); add(sp.k4p); add(sp.k3u);
+  add(sp.nob); add(sp.lastcta); add(sp.block); add(sp.k4r); add(sp.k4g); add(sp.rd); add(sp.k4p); add(sp.k3u);
   add(sp.rowu); add(sp.loopd); add(sp.loopf); add(sp.invmask);
   add(sp.k4b); add(sp.k4b_rb); add(sp.k4b_ns); add(sp.k4b_cb); add(sp.k3rv); add(sp.k3tu);
   k += literal_key(t) + '|';
@@ -1202,6 +1203,19 @@ static CUfunction kernel_for(const Spec& sp, const Tape& t) {
   std::lock_guard<std::mutex> lk(m);
   cache[key] = fn;
   return fn;
+}
+
+// CTAs of 256 threads without dynamic shared memory that an SM holds of a
+// kernel; asked once per kernel (kernels are never unloaded)
+static int resident_ctas(CUfunction fn) {
+  static std::mutex m;
+  static std::unordered_map<CUfunction, int> known;
+  std::lock_guard<std::mutex> lk(m);
+  auto it = known.find(fn);
+  if (it != known.end()) return it->second;
+  int per_sm = 0;
+  check_cu(drv().cuOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0), "occupancy");
+  return known[fn] = std::max(per_sm, 1);
 }
 
 // ============================================================================
@@ -2222,6 +2236,17 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
     sp.k4r = R;
     sp.rd = rdim;
     const int64_t nset = cdiv(KG, GPC);
+    // Rows' loads taken together need registers, so fewer CTAs are resident (4
+    // to 5 of 256 threads an SM, 7 to 8 for the plain loop): where the sets of
+    // columns are a few times the SMs and cannot be split to fit, that costs a
+    // second round ((256, 256, 1024) float32 maximum over axis 1, 1024 sets:
+    // 58 us against 48) and the plain loop stays. With at most 4 sets an SM the
+    // loads decide; with 16 or more they do for sums ((200, 777, 333) float32
+    // 50 -> 43), not for extremes, whose plain loop has 8 CTAs an SM
+    // ((128, 1200, 1024) float32 maximum 95 against 103).
+    const bool fill = tps < 0;
+    sp.k4g = fill && !out && (nset <= 4 * (int64_t)sms || (nset >= 16 * (int64_t)sms && has_sum)) ? 1 : 0;
+    if (fill) tps = RN <= 256 ? 512 : 1024;
     if (tps == 0) {
       // persistent grid: every resident CTA, units of 4R rows split evenly
       sp.k4p = 1;
@@ -2267,12 +2292,33 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
       S = best;
     }
     int64_t C = cdiv(RN, S);
+    CUfunction fn = nullptr;
+    if (sp.k4g && 2 * nset > (sp.vec == 1 ? 8 : 5) * (int64_t)sms) {
+      S = 1;   // two splits of every set would not be resident together (one element a lane: up to 8 CTAs an SM)
+      C = RN;
+    } else if (sp.k4g) {
+      // every CTA resident at once: a second round that a few CTAs fill takes as
+      // long as the first ((1024, 256, 512) int32 sum, 1024 CTAs where 760 fit:
+      // 112 us, 512 CTAs 83). As many splits as fit, in whole trips of
+      // unroll * R rows; more than asked for above only with two trips each and
+      // at least 16 sets of columns, since the merge walks the splits
+      // ((16384, 1024) bfloat16, 152 splits: 30 us, 190: 36)
+      sp.lastcta = lastcta;
+      fn = kernel_for(sp, tape);
+      const int64_t fit = (int64_t)sms * resident_ctas(fn) / nset, trip = (int64_t)unroll * R;
+      S = std::max<int64_t>(1, std::min<int64_t>(fit, nset >= 16 ? std::max<int64_t>(S, RN / (2 * trip)) : S));
+      C = cdiv(cdiv(RN, trip), S) * trip;
+    }
     S = cdiv(RN, C);
     const WordLayout L = word_layout(sp.nops, sp.nd, sp.nscal, sp.nred, sp.ptrmask != 0);
     std::vector<uint64_t> w;
     fill_common_words(s, sp, tape, L, w);
     w[L.nsplit] = (uint64_t)S; w[L.chunk] = (uint64_t)C; w[L.keptn] = (uint64_t)KN; w[L.redn] = (uint64_t)RN;
-    sp.lastcta = (lastcta && S > 1) ? 1 : 0;
+    const int merge = (lastcta && S > 1) ? 1 : 0;
+    if (!fn || merge != sp.lastcta) {
+      sp.lastcta = merge;
+      fn = kernel_for(sp, tape);
+    }
     const size_t pbytes = S > 1 ? (size_t)(S * KN) * 8 * ((has_sum ? 1 : 0) + (has_max ? 2 : 0) + (has_min ? 2 : 0)) : 0;
     uint32_t* cnt = sp.lastcta ? arrival_counters(nset, stream) : nullptr;
     const size_t cbytes = sp.lastcta && !cnt ? ((size_t)nset * 4 + 255) / 256 * 256 : 0;
@@ -2285,10 +2331,10 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
       w[L.aux] = (uint64_t)(uintptr_t)(cnt ? (void*)cnt : (void*)p);
       if (cbytes) check_cuda(cudaMemsetAsync(p, 0, cbytes, stream), "arrival counters");
     }
-    CUfunction fn = kernel_for(sp, tape);
     launch(fn, nset * S, w, stream);
     if (S > 1 && !sp.lastcta) launch_finalize(sp, tape, KN, S, sms, w, stream);
     sp.k4r = 0;
+    sp.k4g = 0;
     sp.rd = 0;
   };
   auto run_k4 = [&](int unroll, int tps, int lastcta) {
@@ -2440,7 +2486,7 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
   // its integer-pipe square root leave the instruction cache, (256, 256, 256)
   // a*b + sqrt|c| - a/2 252 us against 209)
   if (rows_ok && !k4r_off())
-    run_k4(out && tape.compute_dtype == NCA_FLOAT64 ? 102 : 108, k4r_persistent() ? 0 : (RN <= 256 ? 512 : 1024), k4r_lastcta());
+    run_k4(out && tape.compute_dtype == NCA_FLOAT64 ? 102 : 108, k4r_persistent() ? 0 : -1, k4r_lastcta());
   else run_k4(4, 1024, 0);
   return true;
 }
