@@ -115,14 +115,17 @@ unsigned long long* marked_counters(int64_t n, cudaStream_t s);
 uint32_t launch_mark();
 
 // ---- chunk tables of the batched kernels --------------------------------------
-// Bytes per chunk: about 4 chunks for each of `ctas` CTAs, in whole slabs,
-// between 64 and 512 KiB. Larger chunks have fewer ends (trees, counts) and
-// leave more of the last round idle: 2000 arrays, 2.2 GB, at 128 / 256 / 384 /
-// 512 / 1024 KiB 597 / 551 / 530 / 525 / 530 us; 600 arrays through the general
-// form, 0.66 GB, at 64 / 128 / 256 / 384 KiB 254 / 216 / 201 / 197 us.
+// Bytes per chunk: a CTA's share of the batch in whole slabs, between 128 and
+// 384 KiB; 512 KiB from 2 MiB a CTA on. Larger chunks have fewer ends (trees,
+// counts) and leave more of the last round idle: 2000 arrays, 2.2 GB, at 128 /
+// 256 / 384 / 512 / 1024 KiB 597 / 551 / 530 / 525 / 530 us; 600 arrays through
+// the general form, 0.66 GB, at 64 / 128 / 256 / 384 KiB 254 / 216 / 201 / 197.
+// Small batches: 160 arrays (352 KB a CTA) at 64 / 128 / 256 / 384 / 512 KiB
+// 68 / 62 / 56 / 54 / 58 us, 40 arrays at 64 / 128 / 512 KiB 25 / 20 / 33.
 inline long long chunk_bytes_for(long long total, long long ctas, long long slab) {
-  const long long want = total / (ctas * 4) / slab * slab;
-  return std::min<long long>(512 * 1024, std::max<long long>(64 * 1024, want));
+  const long long per = total / ctas;
+  if (per >= 2 * 1024 * 1024) return 512 * 1024;
+  return std::min<long long>(384 * 1024, std::max<long long>(128 * 1024, per / slab * slab));
 }
 // Stable order by descending size, in linear time: 64 classes per power of two.
 template <class C, class F>
