@@ -733,7 +733,7 @@ void run(const nca_view* a, const nca_view* b, const double* w27, double dt, int
 namespace {
 // Arrival counters of kernels whose last CTA merges the partial results, one
 // block of them per stream (see stream_words). Zero when the module loads.
-constexpr int ARR_STREAMS = 64, ARR_N = 16384;
+constexpr int ARR_STREAMS = 64, ARR_N = 4096;
 __device__ uint32_t g_arrivals[ARR_STREAMS][ARR_N];
 __device__ unsigned long long g_marked[ARR_STREAMS][ARR_N];
 }  // namespace

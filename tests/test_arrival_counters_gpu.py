@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 # (shape, axes): a full reduction (one counter), few kept positions, columns
 # (counters per set of columns), and more sets of columns than a stream's block
-# of 16384 counters (16385 * 256 columns of float32)
+# of 16384 counters (16385 * 256 columns of float32: beyond any block)
 CASES = [((64, 4096), None), ((3, 70000), [1]), ((600, 1000), [0]), ((3000, 256), [0])]
 
 
