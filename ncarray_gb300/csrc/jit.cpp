@@ -1972,9 +1972,9 @@ int reduce_out_dtype(int op, int in_dt) {
 // NCA_K4_BULK=1 puts eligible outer reductions on the bulk-staged row-lane
 // form (measured, GB300, CUDA-graph replays: sum over axis 0 of (4096, 16384)
 // float32 0.72 of measured HBM at best over 1-4 column blocks, 2-8 stages and
-// 4-32 rows per stage, against 0.73 for the plain row-lane form; max over axis
-// 1 of (256, 256, 1024) 0.79 against 0.81: the loads in flight are not what
-// bounds these shapes); any NCA_K4_ROWS setting names another form
+// 4-32 rows per stage, against 0.73 for the plain row-lane loop and 0.84 with
+// its rows' loads taken together; max over axis 1 of (256, 256, 1024) 0.79
+// against 0.81); any NCA_K4_ROWS setting names another form
 static bool k4b_on() {
   const char* e = getenv("NCA_K4_BULK");
   const char* r = getenv("NCA_K4_ROWS");
@@ -1995,7 +1995,7 @@ static int k4r_lastcta() {
 }
 // NCA_K4_ROWS=3: the row-lane form on a persistent grid of equal unit ranges
 // (a tuner candidate; measured slower than the splits on (4096, 16384) axis 0,
-// 0.66 against 0.73, and (256, 256, 1024) axis 1, 0.74 against 0.77)
+// 0.66 against 0.84, and (256, 256, 1024) axis 1, 0.74 against 0.81)
 static bool k4r_persistent() {
   const char* e = getenv("NCA_K4_ROWS");
   return e && e[0] == '3';
@@ -2478,10 +2478,8 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
     run_k4(cands[(size_t)best][0], cands[(size_t)best][1], cands[(size_t)best][2]);
     return true;
   }
-  // row-lane form: 8 rows in flight per row lane (the tuner's choice on the
-  // outer-axis benchmarks and C1: max over axis 1 0.77 -> 0.81 of measured);
-  // splits for 1024 threads per SM, 512 for short reduced axes (the tuner's
-  // choices: (4096, 16384) over axis 0 and C1's 128 rows)
+  // row-lane form: 8 rows in flight per row lane (max over axis 1 of (256, 256,
+  // 1024) 0.77 -> 0.81 of measured); the splits are chosen there: -1
   // (stored float64 expressions take 2 rows at a time: 8 copies of a tape with
   // its integer-pipe square root leave the instruction cache, (256, 256, 256)
   // a*b + sqrt|c| - a/2 252 us against 209)
