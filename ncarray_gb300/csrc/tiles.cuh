@@ -149,7 +149,7 @@ tile_prefix_kernel(int ntiles, const long long* __restrict__ cap, const unsigned
 // Elements without a bin count as one more tile behind the others, so nothing
 // branches on them. Waits are bounded (2 s of %globaltimer): on a timeout the
 // CTA records NCA_ERR_TIMEOUT in *status, waits for its copy in flight and
-// stops. Bound: issue and shared-memory latency between the four barriers of a
+// stops. Bound: shared memory (72 % of its data pipe) and the four barriers of a
 // chunk. 2^26 weighted points into 64 tiles 300 -> 237 us (0.75 of the measured
 // copy rate) against a double buffer, 2048-point chunks of 256 threads, 4-byte
 // shared loads, ranks kept in registers and a second scan; 16-byte global loads
