@@ -1909,7 +1909,8 @@ void expr_eval(const Tape& tape, const nca_view* ops, int nops, const nca_view& 
     w[L.nsplit] = (uint64_t)nseg;
     w[L.chunk] = (uint64_t)units;
     groups = units * 32;   // threads
-  } else {
+  } else if (sp.kind == 2) {
+    // (kind 1 decodes no coordinates, and its one dim may be shorter than a vector)
     for (int d = 0; d < s.nd; ++d) {
       int64_t dv = s.shape[d];
       if (d == s.nd - 1) dv /= sp.vec;
