@@ -299,9 +299,12 @@ void launch(ScatterArgs& a, cudaStream_t s) {
   const bool fast = a.nd == 1 && same_src<D>(a.src_dt) && a.dest_n < (1ll << 31) &&
                     a.istr[0] % isz == 0 && a.sstr[0] % (long long)sizeof(D) == 0 &&
                     (uintptr_t)a.idx % isz == 0 && (uintptr_t)a.src % sizeof(D) == 0;
-  auto big = [&](const void* fn) {   // more shared memory than the default limit
+  // more shared memory than the default limit. Always the same value: the limit is
+  // the kernel's on the device, and another thread may be launching it with more
+  // than this call needs
+  auto big = [&](const void* fn) {
     if (bytes > 48 * 1024)
-      nca::check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "smem attribute");
+      nca::check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX_BYTES), "smem attribute");
   };
   if (fast) {
     const int sgn = a.idx_dt == NCA_INT32 ? 1 : 0;

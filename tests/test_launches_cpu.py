@@ -19,3 +19,28 @@ for dt in (DType.float32, DType.int8, DType.float64, DType.bfloat16):
 """
     for dt, shape, n, grid, _ in fake_cuda.run(code, tmp_path):
         assert n == 1 and grid == [1, 1, 1], (dt, shape)
+
+
+def test_scatter_shared_memory_limit_never_falls(built_lib, tmp_path):
+    """The shared-memory limit of a kernel belongs to the device: a call that lowered it to its own need would fail a
+    launch that another thread is about to make with more."""
+    code = """
+result = []
+for dt in (DType.float32, DType.int64):
+    n = 1 << 24
+    for bytes_ in (200 * 1024, 52 * 1024, 120 * 1024, 48 * 1024 + 8):
+        m = bytes_ // nca.dtype.ITEMSIZE[dt]
+        dest, idx, src = array((m,), dt), array((n,), DType.int32), array((n,), dt)
+        for s in (src, array((2 * n,), dt)[::2], array((n,), DType.int16)):   # the fast form, a strided source, a converted one
+            dest.scatter_add(idx, s)
+        result += calls()
+"""
+    calls = fake_cuda.run(code, tmp_path)
+    limits = {}
+    for c in calls:
+        if "smem_limit" in c:
+            assert c["smem_limit"] >= limits.get(c["kernel"], 0), c
+            limits[c["kernel"]] = c["smem_limit"]
+        elif c.get("smem", 0) > 48 * 1024:
+            assert c["smem"] <= limits[c["launch"]], c
+    assert len(limits) >= 4   # both forms of both types took private copies
