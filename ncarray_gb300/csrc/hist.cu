@@ -263,6 +263,9 @@ tile_combine_kernel(long long nbins, int G, const long long* __restrict__ PV,
   // weight sums as float-float pairs: the float64 adds and conversions of every
   // piece were most of the pass on this card
   float wh[4] = {0.f, 0.f, 0.f, 0.f}, wl[4] = {0.f, 0.f, 0.f, 0.f};
+  // past the last bin the pieces hold whatever the scratch held before: such
+  // values are neither stored nor asked whether they are finite
+  const int nb = (int)(nbins - bin < 4 ? nbins - bin : 4);
   bool finite = true;
   auto slot_of = [&](int g) { return (long long)(g + t) * TB + (bin - (long long)t * TB); };
   auto add = [&](int g) {
@@ -270,10 +273,10 @@ tile_combine_kernel(long long nbins, int G, const long long* __restrict__ PV,
     cn[0] += c.x; cn[1] += c.y; cn[2] += c.z; cn[3] += c.w;
     if (WEIGHTED) {
       const float4 a = *reinterpret_cast<const float4*>(ps + slot_of(g)), e = *reinterpret_cast<const float4*>(pe + slot_of(g));
-      finite &= ff_add(wh[0], wl[0], a.x, e.x);
-      finite &= ff_add(wh[1], wl[1], a.y, e.y);
-      finite &= ff_add(wh[2], wl[2], a.z, e.z);
-      finite &= ff_add(wh[3], wl[3], a.w, e.w);
+      finite &= ff_add(wh[0], wl[0], a.x, e.x) | (0 >= nb);
+      finite &= ff_add(wh[1], wl[1], a.y, e.y) | (1 >= nb);
+      finite &= ff_add(wh[2], wl[2], a.z, e.z) | (2 >= nb);
+      finite &= ff_add(wh[3], wl[3], a.w, e.w) | (3 >= nb);
     }
   };
   // (an empty range stored no piece)
@@ -301,13 +304,13 @@ tile_combine_kernel(long long nbins, int G, const long long* __restrict__ PV,
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       cn[k] += scn[u][q][k];
-      if (WEIGHTED) finite &= ff_add(wh[k], wl[k], sw[u][q][k].x, sw[u][q][k].y);
+      if (WEIGHTED) finite &= ff_add(wh[k], wl[k], sw[u][q][k].x, sw[u][q][k].y) | (k >= nb);
     }
   if (s_bad) finite = false;
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    if (bin + k >= nbins) break;
+    if (k >= nb) break;
     counts[bin + k] += cn[k];
     if (WEIGHTED) {
       const float w0 = wsum[bin + k];
