@@ -8,7 +8,7 @@
 // and the point is kept only if 0 <= fx < nbx and 0 <= fy < nby (NaN dropped).
 // counts (uint64) are exact; weights are summed per bin with float32 partial
 // sums whose rounding errors are collected exactly (compensated), combined as
-// float-float pairs, and added to the float32 output once at the end.
+// sums of three floats, and added to the float32 output once at the end.
 //
 // A bin grid of more than a few thousand bins does not fit in shared memory
 // and global atomics on it run at the L2 atomic rate, far below HBM speed.
@@ -28,7 +28,7 @@
 //      compensation terms: the value returned by the float atomic gives the
 //      exact rounding error of each addition via TwoSum) and stores the piece;
 //   4. combine: every bin adds its tile's pieces in a fixed order (uint64
-//      counts, float-float weights) to the outputs.
+//      counts, three-float weights) to the outputs.
 // Passes 1 and 2 are in tiles.cuh.
 // Small inputs and grids with too many tiles use direct global atomics.
 #include <cuda_runtime.h>
@@ -220,14 +220,36 @@ tile_accumulate_kernel(int nv, const long long* __restrict__ off, const long lon
   }
 }
 
-// (hi, lo) += (a, e) as float-float pairs: the rounding error of hi + a is kept
-// exactly in lo; false when the sum is not finite
-__device__ __forceinline__ bool ff_add(float& hi, float& lo, float a, float e) {
-  const float s = __fadd_rn(hi, a), bb = __fsub_rn(s, hi);
-  lo = __fadd_rn(__fadd_rn(lo, e), __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bb)), __fsub_rn(a, bb)));
-  hi = s;
-  return fabsf(s) < __int_as_float(0x7f800000);
-}
+// A weight sum as three floats: additions to the first two keep their rounding
+// errors exactly, the third collects what the second loses. With n terms and
+// partial sums up to M it is off by at most about n^3 M 2^-72, less than the
+// n M 2^-53 of a float64 sum for n up to 700; a bin has at most a piece per
+// accumulating CTA, one an SM.
+struct Sum3 {
+  float hi, mid, lo;
+  // a = rn(a + b); returns the error of that addition
+  static __device__ __forceinline__ float two_sum(float& a, float b) {
+    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+    const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    a = s;
+    return e;
+  }
+  __device__ __forceinline__ void add(float a, float b) {
+    const float ea = two_sum(hi, a), eb = two_sum(mid, b);
+    lo = __fadd_rn(lo, __fadd_rn(eb, two_sum(mid, ea)));
+  }
+  __device__ __forceinline__ void add(const Sum3& o) {
+    add(o.hi, o.mid);
+    lo = __fadd_rn(lo, o.lo);
+  }
+  // a sum that left float32's range stays outside it
+  __device__ __forceinline__ bool finite() const { return fabsf(hi) < __int_as_float(0x7f800000); }
+  // the sum as a float, off by half a unit in the last place
+  __device__ __forceinline__ float get() {
+    const float e = two_sum(hi, mid);
+    return __fadd_rn(hi, __fadd_rn(e, lo));
+  }
+};
 
 // ---- pass 4: add the pieces of every bin's tile to the outputs ----------------------
 // A block takes 4 * THREADS / CG bins of one tile, four a thread, and splits the
@@ -235,9 +257,12 @@ __device__ __forceinline__ bool ff_add(float& hi, float& lo, float a, float e) {
 // tiles one has pieces from many CTAs, and a loop over them is a chain of load
 // latency (CG = 4 from 8 pieces a tile on: 64 x 64 bins, 2^20 points 61 -> 44 us
 // a call; 1024 x 1024 bins have 2-3 pieces a tile, CG = 1). The sharing CTAs
-// come from the prefix pass and the weights are float-float pairs: 64-bit
-// divisions and float64 adds and conversions per bin were most of the pass
-// (50-65 us for 1024 x 1024 weighted bins, now 20-22).
+// come from the prefix pass and the weights are sums of three floats (Sum3):
+// 64-bit divisions and float64 adds and conversions per bin were most of the
+// pass (50-65 us for 1024 x 1024 weighted bins, 20-22 with pairs of floats;
+// with three a call takes the same time within 1 us). The output's old value is
+// one more term: 2^20 points added to 2048 x 2048 bins 160 -> 134 us a call
+// without float64 arithmetic for it.
 template <bool WEIGHTED, int CG>
 __global__ void __launch_bounds__(THREADS)
 tile_combine_kernel(long long nbins, int G, const long long* __restrict__ PV,
@@ -246,9 +271,10 @@ tile_combine_kernel(long long nbins, int G, const long long* __restrict__ PV,
                     float* __restrict__ wsum, int ntiles, const int2* __restrict__ ctas) {
   static_assert(TB % (4 * THREADS) == 0, "a block's bins lie in one tile");
   constexpr int Q = THREADS / CG;   // threads per group, four bins each
+  constexpr int LOADS = CG > 1 ? 4 : 1;   // (2 pieces a tile with CG = 1: nothing to batch)
   __shared__ int s_bad;
   __shared__ unsigned long long scn[CG > 1 ? CG - 1 : 1][CG > 1 ? Q : 1][4];
-  __shared__ float2 sw[CG > 1 ? CG - 1 : 1][CG > 1 ? Q : 1][4];
+  __shared__ Sum3 sw[CG > 1 && WEIGHTED ? CG - 1 : 1][CG > 1 && WEIGHTED ? Q : 1][4];
   const int q = threadIdx.x % Q, grp = threadIdx.x / Q;
   const long long bin0 = (long long)blockIdx.x * 4 * Q;
   const int t = (int)(bin0 / TB);
@@ -260,53 +286,65 @@ tile_combine_kernel(long long nbins, int G, const long long* __restrict__ PV,
   }
   const long long bin = bin0 + 4 * q;
   unsigned long long cn[4] = {0, 0, 0, 0};
-  // weight sums as float-float pairs: the float64 adds and conversions of every
-  // piece were most of the pass on this card
-  float wh[4] = {0.f, 0.f, 0.f, 0.f}, wl[4] = {0.f, 0.f, 0.f, 0.f};
+  Sum3 ws[4] = {};
   // past the last bin the pieces hold whatever the scratch held before: such
   // values are neither stored nor asked whether they are finite
   const int nb = (int)(nbins - bin < 4 ? nbins - bin : 4);
-  bool finite = true;
   auto slot_of = [&](int g) { return (long long)(g + t) * TB + (bin - (long long)t * TB); };
-  auto add = [&](int g) {
-    const uint4 c = *reinterpret_cast<const uint4*>(pc + slot_of(g));
-    cn[0] += c.x; cn[1] += c.y; cn[2] += c.z; cn[3] += c.w;
+  uint4 pcv[LOADS];
+  float4 psv[LOADS], pev[LOADS];
+  auto load = [&](int u, int g) {
+    pcv[u] = *reinterpret_cast<const uint4*>(pc + slot_of(g));
     if (WEIGHTED) {
-      const float4 a = *reinterpret_cast<const float4*>(ps + slot_of(g)), e = *reinterpret_cast<const float4*>(pe + slot_of(g));
-      finite &= ff_add(wh[0], wl[0], a.x, e.x) | (0 >= nb);
-      finite &= ff_add(wh[1], wl[1], a.y, e.y) | (1 >= nb);
-      finite &= ff_add(wh[2], wl[2], a.z, e.z) | (2 >= nb);
-      finite &= ff_add(wh[3], wl[3], a.w, e.w) | (3 >= nb);
+      psv[u] = *reinterpret_cast<const float4*>(ps + slot_of(g));
+      pev[u] = *reinterpret_cast<const float4*>(pe + slot_of(g));
+    }
+  };
+  auto add = [&](int u) {
+    cn[0] += pcv[u].x; cn[1] += pcv[u].y; cn[2] += pcv[u].z; cn[3] += pcv[u].w;
+    if (WEIGHTED) {
+      ws[0].add(psv[u].x, pev[u].x);
+      ws[1].add(psv[u].y, pev[u].y);
+      ws[2].add(psv[u].z, pev[u].z);
+      ws[3].add(psv[u].w, pev[u].w);
     }
   };
   // (an empty range stored no piece)
   auto empty = [&](int g) { return R < G && range_start(R, g, G) == range_start(R, g + 1, G); };
-  if (R >= G) {
-#pragma unroll 8
-    for (int g = s_first + grp; g <= s_last; g += CG) add(g);   // several pieces' loads in flight
-  } else {
-    for (int g = s_first + grp; g <= s_last; g += CG)
-      if (!empty(g)) add(g);
-  }
+  int g = s_first + grp;
+  if (R >= G)
+    for (; g + (LOADS - 1) * CG <= s_last; g += LOADS * CG) {   // LOADS pieces' loads in flight
+#pragma unroll
+      for (int u = 0; u < LOADS; ++u) load(u, g + u * CG);
+#pragma unroll
+      for (int u = 0; u < LOADS; ++u) add(u);
+    }
+  for (; g <= s_last; g += CG)
+    if (!empty(g)) { load(0, g); add(0); }
+  bool finite = true;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) finite &= ws[k].finite() | (k >= nb);
   if (CG > 1) {
-  if (!finite) s_bad = 1;
-  if (grp > 0) {
+    if (!finite) s_bad = 1;
+    if (grp > 0) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      scn[grp - 1][q][k] = cn[k];
-      if (WEIGHTED) sw[grp - 1][q][k] = make_float2(wh[k], wl[k]);
+      for (int k = 0; k < 4; ++k) {
+        scn[grp - 1][q][k] = cn[k];
+        if (WEIGHTED) sw[grp - 1][q][k] = ws[k];
+      }
     }
-  }
-  __syncthreads();
-  if (grp > 0) return;
+    __syncthreads();
+    if (grp > 0) return;
 #pragma unroll
-  for (int u = 0; u < CG - 1; ++u)
+    for (int u = 0; u < CG - 1; ++u)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      cn[k] += scn[u][q][k];
-      if (WEIGHTED) finite &= ff_add(wh[k], wl[k], sw[u][q][k].x, sw[u][q][k].y) | (k >= nb);
-    }
-  if (s_bad) finite = false;
+      for (int k = 0; k < 4; ++k) {
+        cn[k] += scn[u][q][k];
+        if (WEIGHTED) ws[k].add(sw[u][q][k]);
+      }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) finite &= ws[k].finite() | (k >= nb);
+    if (s_bad) finite = false;
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -315,11 +353,15 @@ tile_combine_kernel(long long nbins, int G, const long long* __restrict__ PV,
     if (WEIGHTED) {
       const float w0 = wsum[bin + k];
       double d = wacc[bin + k];
-      if (finite && w0 == 0.f && d == 0.0) {
-        wsum[bin + k] = __fadd_rn(wh[k], wl[k]);
-        continue;
+      if (finite && d == 0.0) {   // the value that is there is one more term
+        Sum3 all = ws[k];
+        all.add(w0, 0.f);
+        if (all.finite()) {
+          wsum[bin + k] = all.get();
+          continue;
+        }
       }
-      double p = (double)wh[k] + (double)wl[k];
+      double p = ((double)ws[k].hi + (double)ws[k].mid) + (double)ws[k].lo;
       if (!finite) {   // sums beyond float32: the pieces again in float64
         p = 0.0;
         for (int g = s_first; g <= s_last; ++g)
