@@ -659,22 +659,30 @@ void launch_one(const Grid3& src, const Grid3& dst, const Weights<T>& W, int mod
   count_launch();
 }
 
+// z chunks of a three-step pass: one CTA per SM at a time, and every chunk
+// marches T3_LAG + 2 planes more than it stores, so the split with the fewest
+// planes end to end. Returns those planes; zt and rounds of resident CTAs.
+template <int NW, int R>
+int64_t split3(const Grid3& g, int sms, int& zt, int64_t& rounds) {
+  const int64_t tiles = (int64_t)((g.nx + T3_TX - 1) / T3_TX) * ((g.ny + T3<NW, R>::TY - 1) / T3<NW, R>::TY);
+  int64_t best = -1;
+  for (int c = 1; c <= g.nz && c <= 4 * sms; ++c) {
+    const int d = (g.nz + c - 1) / c;
+    const int64_t r = (tiles * ((g.nz + d - 1) / d) + sms - 1) / sms, cost = r * (d + T3_LAG + 2);
+    if (best < 0 || cost < best) { best = cost; zt = d; rounds = r; }
+  }
+  return best;
+}
+
 template <int MODE, int NW, int R>
 void launch3_as(const Grid3& src, const Grid3& dst, const Weights<float>& W, cudaStream_t s) {
   using namespace nca;
   CUtensorMap m;
   encode_box<float>(&m, src, T3_EX, T3<NW, R>::EY);
-  const int sms = sm_count(current_device());
   const int tx = (src.nx + T3_TX - 1) / T3_TX, ty = (src.ny + T3<NW, R>::TY - 1) / T3<NW, R>::TY;
-  // z chunks: one CTA per SM at a time, and every chunk marches 8 planes more
-  // than it stores, so take the split with the fewest planes end to end
-  int64_t best = -1;
   int zt = src.nz;
-  for (int c = 1; c <= src.nz && c <= 4 * sms; ++c) {
-    const int d = (src.nz + c - 1) / c;
-    const int64_t cost = (((int64_t)tx * ty * ((src.nz + d - 1) / d) + sms - 1) / sms) * (d + T3_LAG + 2);
-    if (best < 0 || cost < best) { best = cost; zt = d; }
-  }
+  int64_t rounds = 1;
+  split3<NW, R>(src, sm_count(current_device()), zt, rounds);
   auto two = [](float v) { return make_float2(v, v); };
   Pairs p{};
   p.dt = two(W.dt);
@@ -690,6 +698,36 @@ void launch3_as(const Grid3& src, const Grid3& dst, const Weights<float>& W, cud
   fn<<<dim3(tx, ty, (src.nz + zt - 1) / zt), 32 * NW, T3<NW, R>::SMEM, s>>>(m, (float*)dst.mut, src.nx, src.ny, src.nz, zt, p);
   check_cuda(cudaGetLastError(), "stencil launch");
   count_launch();
+}
+
+// Whether a three-step pass is shorter than three single steps: both are
+// estimated, in us. A pass takes its planes end to end, 0.93 us each for 7
+// points and 0.82 for 27 (1.13 and 0.94 where only one round of CTAs runs, which
+// nothing overlaps). A single step takes the time of one CTA's march, or of all
+// CTAs (several an SM), or of the bytes, whichever is longest. What tiles of 120
+// columns and 36 or 18 rows waste on a narrow grid, and the 10 extra planes of
+// a chunk on a flat one, decides: three steps against one pass, 7 points / 27,
+// (1, 2048, 2048) 43 against 74 / 55 against 129; (4, 2048, 2048) 80, 92 / 103,
+// 156; (8, 2048, 2048) 135, 123 / 160, 207; (16, 2048, 2048) 261, 183 / 302, 307;
+// (8, 8, 100000) 49, 103 / 68, 89; (512, 512, 32) 67, 70 / 92, 107; (64, 64, 64)
+// 25, 14 / 31, 12; (512, 512, 512) 511, 300 / 510, 481. Of 74 grids measured the
+// rule takes the slower form for four, by 5 % or less in all but one
+// ((512, 512, 132) with 27 points keeps single steps: 221 against 209).
+bool three_pays(const Grid3& g, int mode, int sms, int tile, int zt1) {
+  const bool star = mode == 1;
+  int zt = g.nz;
+  int64_t rounds = 1;
+  const double planes = (double)(star ? split3<14, 3>(g, sms, zt, rounds) : split3<12, 2>(g, sms, zt, rounds));
+  const double pass = 1.5 + planes * (star ? 0.93 + 0.2 / (double)rounds : 0.82 + 0.12 / (double)rounds);
+  const int d = std::min(zt1, g.nz) + 2;
+  const int64_t n = (int64_t)((g.nx + kTiles[tile][0] - 1) / kTiles[tile][0]) *
+                    ((g.ny + kTiles[tile][1] - 1) / kTiles[tile][1]) * ((g.nz + zt1 - 1) / zt1);
+  const bool few = n <= 4 * (int64_t)sms;
+  const double r = few ? (double)((n + sms - 1) / sms) : (double)n / sms;
+  const double march = star ? 2.6 + 0.35 * d : 2.9 + 0.4 * d;
+  const double issue = (star ? (few ? 0.165 : 0.155) : (few ? 0.225 : 0.187)) * d * r;
+  const double bytes = (double)g.nx * g.ny * g.nz * 8.0 / 6.7e6;
+  return pass < 3.0 * std::max(march, std::max(issue, bytes));
 }
 
 void launch3(const Grid3& src, const Grid3& dst, const Weights<float>& W, int mode, cudaStream_t s) {
@@ -708,11 +746,16 @@ void run(const nca_view* a, const nca_view* b, const double* w27, double dt, int
   const char *pa = (const char*)ga.base, *pb = (const char*)gb.base;
   if (pa < pb + bytes && pb < pa + bytes) fail(NCA_ERR_INVALID, "stencil source and destination overlap");
   const int mode = star7(w27) ? 1 : isotropic27(w27) ? 2 : 0;
-  // steps 1 .. iters-1 three at a time where the three-step kernel applies
+  // steps 1 .. iters-1 three at a time where the three-step kernel applies and pays
   // (each pass moves the result to the other grid, and three single steps do
   // too); the last step runs alone, so that afterwards the two grids hold the
   // last two iterates, as when every step runs alone
-  const bool three = ga.dtype == NCA_FLOAT32 && mode != 0 && tma_ok(ga) && tma_ok(gb);
+  bool three = ga.dtype == NCA_FLOAT32 && mode != 0 && iters > T3_K && tma_ok(ga) && tma_ok(gb);
+  if (three) {
+    int tile = 0, zt = 8;
+    tma_schedule<float>(ga, gb, make_weights<float>(w27, dt), mode, s, tile, zt);
+    three = three_pays(ga, mode, sm_count(current_device()), tile, zt);
+  }
   bool from_a = true;
   for (int it = 0; it < iters; from_a = !from_a) {
     const Grid3& src = from_a ? ga : gb;

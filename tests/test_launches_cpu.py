@@ -44,3 +44,21 @@ for dt in (DType.float32, DType.int64):
         elif c.get("smem", 0) > 48 * 1024:
             assert c["smem"] <= limits[c["launch"]], c
     assert len(limits) >= 4   # both forms of both types took private copies
+
+
+def test_three_step_stencil_only_where_it_pays(built_lib, tmp_path):
+    """Flat and narrow grids keep single steps; (steps - 1) // 3 passes elsewhere."""
+    code = """
+from ncarray_gb300.stencil import Stencil3D, laplacian7, laplacian27
+result = []
+for points, w in ((7, laplacian7()), (27, laplacian27())):
+    for shape in ((1, 2048, 2048), (2, 2048, 2048), (4, 2048, 2048), (1, 300000, 4), (8, 8, 100000), (64, 4096, 8), (1, 8192, 8192),
+                  (512, 512, 512), (64, 64, 64), (200, 300, 400), (256, 36, 120)):
+        a, b = array(shape, DType.float32), array(shape, DType.float32)
+        Stencil3D(w, 0.1).iterate(a, b, 11)
+        result.append([points, shape, ["tma3" in c["launch"] for c in launches()]])
+"""
+    flat = {(1, 2048, 2048), (2, 2048, 2048), (4, 2048, 2048), (1, 300000, 4), (8, 8, 100000), (64, 4096, 8), (1, 8192, 8192)}
+    for points, shape, three in fake_cuda.run(code, tmp_path):
+        want = [False] * 11 if tuple(shape) in flat else [True] * 3 + [False] * 2
+        assert three == want, (points, shape)
