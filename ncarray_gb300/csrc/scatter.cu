@@ -45,6 +45,7 @@ struct ScatterArgs {
   long long dest_stride;  // bytes
   int nd;                 // canonical dims (1..NCA_MAX_NDIM)
   int idx_dt, src_dt;
+  int runs_direct;        // runs of equal indices go to global memory (scatter_fast_kernel)
   long long shape[NCA_MAX_NDIM];
   long long istr[NCA_MAX_NDIM];
   long long sstr[NCA_MAX_NDIM];
@@ -173,37 +174,75 @@ __global__ void __launch_bounds__(SMEM ? 1024 : THREADS) scatter_add_kernel(Scat
   }
 }
 
+template <class D>
+__device__ __forceinline__ D warp_sum(D v) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+  return v;
+}
+
 // The common case in one pass with more loads in flight: 1-D views, the
 // source already of the destination's type, indices of 32 or 64 bits, a
 // destination below 2^31 entries (32-bit match keys). A warp takes 32 * U
 // consecutive elements per trip (U loads of each array in flight per thread,
-// the source loaded without waiting for its index); grouping and atomics as
-// in scatter_add_kernel.
+// the source loaded without waiting for its index).
+//
+// Grouping a warp's equal indices as scatter_add_kernel does costs about 75
+// clocks per SM and 32 elements, more than the atomics of distinct ones, so a
+// warp groups one trip in 16 and the others only when that one found repeats:
+//   - atomics on global memory (LOOP): any repeat. One address takes an atomic
+//     in 1.3 ns, so an index with 1 % of 2^26 elements alone takes longer than
+//     grouping all of them. An index that repeats is first taken out altogether:
+//     the warp keeps it as its hot entry, adds its elements in registers and
+//     issues one atomic at the end or when a sampled trip lacks it (the warps
+//     of a CTA tell each other, since a rare one is seen by few);
+//   - private copies (PRIVATE): 5 lanes with repeats (float64: or an index
+//     three times in a load, whose serial adds cost more). Sampled indices that
+//     repeat in runs of neighbours (sorted input) go to global memory unless
+//     the copies were privatised for the group sums too (runs_direct): a group
+//     is one atomic there that nothing waits for;
+//   - a trip of one entry is one sum and one atomic.
+// ONE_TRIP is for inputs that the grid covers in one trip: it groups always and
+// has none of the choices, whose instructions cost a short kernel 2 us.
+// 2^26 float32 elements, us, always grouping -> now: into 2^20 entries 525 ->
+// 346 (L2 atomics, 194 G/s), 12000 527 -> 151, 50000 525 -> 154; with 1 / 5 / 50
+// % in one index of 2^20 954 -> 411, 2631 -> 389, 3225 -> 316; a power law 6995
+// -> 6947; sorted 222 -> 211, in fours 232 -> 243. 2^23 into 12000 to 50000: 29
+// us sorted, 31 in fours, now 31 and 35-37 through private copies. float64 into
+// 12000: 690 -> 223, sorted 683 -> 334; into 1000 with 5 % in one index 907 ->
+// 1068 (the price of 578 -> 360 without one).
 constexpr int U = 4;
+enum Form { ONE_TRIP, LOOP, PRIVATE };
 
-template <class D, class IW, bool SMEM>
-__global__ void __launch_bounds__(SMEM ? 1024 : THREADS) scatter_fast_kernel(ScatterArgs a, int idx_signed) {
-  const int nthr = SMEM ? (int)blockDim.x : THREADS;
+template <class D, class IW, int FORM>
+__global__ void __launch_bounds__(FORM == PRIVATE ? 1024 : THREADS) scatter_fast_kernel(ScatterArgs a) {
+  constexpr bool PRIV = FORM == PRIVATE, HOT = FORM == LOOP;
+  const int nthr = PRIV ? (int)blockDim.x : THREADS;
   extern __shared__ __align__(16) unsigned char sm_raw[];
+  __shared__ int s_hot;   // the last hot entry that a warp of this CTA found
   D* priv = reinterpret_cast<D*>(sm_raw);
-  if (SMEM) {
+  if (PRIV)
     for (long long b = threadIdx.x; b < a.dest_n; b += nthr) priv[b] = D(0);
-    __syncthreads();
-  }
+  if (HOT && threadIdx.x == 0) s_hot = -1;
+  if (PRIV || HOT) __syncthreads();
   const IW* idx = reinterpret_cast<const IW*>(a.idx);
   const D* src = reinterpret_cast<const D*>(a.src);
   const long long ist = a.istr[0] / (long long)sizeof(IW), sst = a.sstr[0] / (long long)sizeof(D);
   const int lane = threadIdx.x & 31;
   const long long stride = (long long)gridDim.x * nthr * U;
-  // Grouping a warp's equal indices costs about 75 clocks per SM and 32
-  // elements, more than the atomics of distinct ones, so a warp groups one trip
-  // in 16 and the others only when 5 lanes of that trip held an element whose
-  // index repeats in its load (an index that takes 7 % of the elements). 2^26 float32 elements, us before -> now: into 2^20
-  // entries 527 -> 367 (L2 atomics, 183 G/s), 12000 528 -> 163 and 50000 527 ->
-  // 165 (private copies, shared-memory atomics); a skewed power law is grouped
-  // as before (2^24: 1205 us), sorted indices too (16 repeats each, 60.5 -> 65:
-  // the price of the choice).
-  bool group = true;
+  // (warp-uniform, as every condition around a warp's shuffles below)
+  bool group = true, runs = false;
+  int hot = -1;
+  D acc = D(0);
+  auto put = [&](int t, D s, bool global) {
+    if (PRIV && !global) atomic_add<D>(priv + t, s);
+    else atomic_add<D>(reinterpret_cast<D*>(a.dest + (long long)t * a.dest_stride), s);
+  };
+  auto flush = [&] {
+    const D s = warp_sum(acc);
+    if (lane == 0 && s != D(0)) put(hot, s, true);
+    acc = D(0);
+  };
   int trip = 0;
   for (long long base = ((long long)blockIdx.x * nthr + (threadIdx.x & ~31)) * U; base < a.n; base += stride, ++trip) {
     IW raw[U];
@@ -211,41 +250,73 @@ __global__ void __launch_bounds__(SMEM ? 1024 : THREADS) scatter_fast_kernel(Sca
 #pragma unroll
     for (int k = 0; k < U; ++k) {
       const long long i = base + k * 32 + lane;
-      raw[k] = (IW)0;
+      raw[k] = ~(IW)0;
       v[k] = D(0);
       if (i < a.n) {
         raw[k] = idx[i * ist];
         v[k] = src[i * sst];
       }
     }
-    long long t[U];
+    // entry of each element, -1 where dropped (a negative index is a large unsigned one)
+    int t[U];
 #pragma unroll
-    for (int k = 0; k < U; ++k) {
-      if (sizeof(IW) == 4) t[k] = idx_signed ? (long long)(int)(unsigned)raw[k] : (long long)(unsigned)raw[k];
-      else t[k] = (long long)(unsigned long long)raw[k];   // uint64 >= 2^63 reads negative: dropped
-      if (base + k * 32 + lane >= a.n || t[k] >= a.dest_n) t[k] = -1;
+    for (int k = 0; k < U; ++k) t[k] = raw[k] < (IW)a.dest_n ? (int)raw[k] : -1;
+    bool seen = false;
+    if (HOT) {
+      if (hot < 0) hot = __shfl_sync(0xffffffffu, *(volatile int*)&s_hot, 0);
+#pragma unroll
+      for (int k = 0; k < U; ++k) seen |= t[k] == hot && hot >= 0;
+      seen = __any_sync(0xffffffffu, seen);
+      if (seen) {   // (a float64 addition costs its pipe even where no lane takes it)
+#pragma unroll
+        for (int k = 0; k < U; ++k)
+          if (t[k] == hot) {
+            acc += v[k];
+            t[k] = -1;
+          }
+      }
     }
-    auto put = [&](int k, D s) {
-      if (SMEM) atomic_add<D>(priv + t[k], s);
-      else atomic_add<D>(reinterpret_cast<D*>(a.dest + t[k] * a.dest_stride), s);
-    };
-    if (!group && (trip & 15) != 0) {
+    const bool sample = FORM != ONE_TRIP && (trip & 15) == 0;
+    if (FORM != ONE_TRIP && !group && !sample) {
 #pragma unroll
       for (int k = 0; k < U; ++k)
-        if (t[k] >= 0) put(k, v[k]);
+        if (t[k] >= 0) put(t[k], v[k], false);
       continue;
     }
-    bool repeated = false;
+    if (FORM != ONE_TRIP) {   // one entry takes the whole trip
+      const int first = __shfl_sync(0xffffffffu, t[0], 0);
+      bool same = first >= 0;
+#pragma unroll
+      for (int k = 0; k < U; ++k) same &= t[k] == first;
+      if (__all_sync(0xffffffffu, same)) {
+        D s = v[0];
+#pragma unroll
+        for (int k = 1; k < U; ++k) s += v[k];
+        s = warp_sum(s);
+        if (lane == 0) put(first, s, false);
+        continue;
+      }
+    }
+    int repeated = -1;
+    bool apart = false, thrice = false;   // equal indices that are not neighbours; three of them in a load
+    unsigned peers[U];
+    auto match = [&](int k) {   // dropped elements stay alone
+      peers[k] = __match_any_sync(0xffffffffu, t[k] >= 0 ? (unsigned)t[k] : 0x80000000u + (unsigned)lane);
+    };
+    if (!PRIV) {   // all matches first: 242 us against 255 in fours of 2^26; private copies have no registers for it
+#pragma unroll
+      for (int k = 0; k < U; ++k) match(k);
+    }
 #pragma unroll
     for (int k = 0; k < U; ++k) {
-      const bool ok = t[k] >= 0;
-      const unsigned key = ok ? (unsigned)t[k] : 0x80000000u + (unsigned)lane;   // invalid lanes stay alone
-      const unsigned peers = __match_any_sync(0xffffffffu, key);
-      D s = ok ? v[k] : D(0);
-      const unsigned above = peers & ~((2u << lane) - 1u);
+      if (PRIV) match(k);
+      D s = v[k];
+      const unsigned above = peers[k] & ~((2u << lane) - 1u);
       int next = above ? __ffs(above) - 1 : lane;
       bool has = above != 0;
-      repeated |= has;
+      if (has) repeated = t[k];
+      if (PRIV) apart |= next > lane + 1;
+      if (PRIV && sizeof(D) == 8) thrice |= __popc(peers[k]) >= 3;
       if (__any_sync(0xffffffffu, has)) {
 #pragma unroll
         for (int r = 0; r < 5; ++r) {
@@ -255,11 +326,29 @@ __global__ void __launch_bounds__(SMEM ? 1024 : THREADS) scatter_fast_kernel(Sca
           if (has) { s += ov; next = onext; has = ohas; }
         }
       }
-      if (ok && (peers & ((1u << lane) - 1u)) == 0) put(k, s);
+      if (t[k] >= 0 && (peers[k] & ((1u << lane) - 1u)) == 0) put(t[k], s, runs);
     }
-    if ((trip & 15) == 0) group = __popc(__ballot_sync(0xffffffffu, repeated)) >= 5;
+    if (sample) {
+      const unsigned any = __ballot_sync(0xffffffffu, repeated >= 0);
+      if (PRIV) {
+        const bool parted = __any_sync(0xffffffffu, apart), three = __any_sync(0xffffffffu, thrice);
+        group = __popc(any) >= 5 || three;
+        runs = a.runs_direct && __popc(any) >= 16 && !parted;
+      } else {
+        group = any != 0;
+        if (hot >= 0 && !seen) {   // gone cold
+          flush();
+          hot = -1;
+        }
+        if (hot < 0 && any) {
+          hot = __shfl_sync(0xffffffffu, repeated, __ffs(any) - 1);
+          if (lane == 0) atomicExch(&s_hot, hot);
+        }
+      }
+    }
   }
-  if (SMEM) {
+  if (HOT && hot >= 0) flush();
+  if (PRIV) {
     __syncthreads();
     for (long long b = threadIdx.x; b < a.dest_n; b += nthr) {
       const D v = priv[b];
@@ -286,15 +375,22 @@ void launch(ScatterArgs& a, cudaStream_t s) {
   const long long bytes = a.dest_n * (long long)sizeof(D);
   long long blocks = (a.n + THREADS - 1) / THREADS;
   // privatise when the destination fits and an element comes per two entries that
-  // the CTAs flush (coalesced atomics, about a tenth of a scattered one each): 4
-  // CTAs of 256 threads per SM up to 48 KB, 2 of 512 up to 100 KB, else 1 of
-  // 1024. 2^23 float32 elements into 6000 entries 242 -> 34 us, 25000 75 -> 30,
-  // 50000 69 -> 32; 2^20 into 6000 34 -> 16; 2^23 float64 into 12000 81 -> 46
-  auto pays = [&](int per_sm) { return 2 * a.n >= (long long)sms * per_sm * a.dest_n; };
+  // the CTAs flush (coalesced atomics, about a tenth of a scattered one each;
+  // 8-byte entries, whose adds are loops, want three elements per four): 4 CTAs
+  // of 256 threads per SM up to 48 KB, 2 of 512 up to 100 KB, else 1 of 1024.
+  // 2^23 float32 elements into 6000 entries 144 -> 30 us, 25000 76 -> 28, 50000
+  // 68 -> 27; 2^20 into 6000 22 -> 13, 12000 13.6 -> 12.6; 2^23 float64 into
+  // 12000 81 -> 45, 2^20 would be 15 -> 17
+  auto pays = [&](int per_sm) {
+    const long long flushed = (long long)sms * per_sm * a.dest_n;
+    return sizeof(D) == 4 ? 2 * a.n >= flushed : 4 * a.n >= 3 * flushed;
+  };
   const int pct = bytes <= 48 * 1024 && pays(4) ? 4 : bytes <= 100 * 1024 && pays(2) ? 2 : 1;
   const int pthreads = 1024 / pct;
   const long long priv_ctas = (long long)sms * pct;
   const bool smem = bytes <= SMEM_MAX_BYTES && pays(pct);
+  // few entries with many elements each: group sums too are better off in the copies
+  a.runs_direct = !(bytes <= 48 * 1024 && a.n >= 16ll * sms * a.dest_n);
   const int isz = (a.idx_dt == NCA_INT64 || a.idx_dt == NCA_UINT64) ? 8 : 4;
   const bool fast = a.nd == 1 && same_src<D>(a.src_dt) && a.dest_n < (1ll << 31) &&
                     a.istr[0] % isz == 0 && a.sstr[0] % (long long)sizeof(D) == 0 &&
@@ -307,18 +403,24 @@ void launch(ScatterArgs& a, cudaStream_t s) {
       nca::check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX_BYTES), "smem attribute");
   };
   if (fast) {
-    const int sgn = a.idx_dt == NCA_INT32 ? 1 : 0;
     long long fb = (a.n + (long long)THREADS * U - 1) / ((long long)THREADS * U);
     if (smem) {
       fb = std::min(fb, priv_ctas);
-      big(isz == 4 ? (const void*)scatter_fast_kernel<D, unsigned, true>
-                   : (const void*)scatter_fast_kernel<D, unsigned long long, true>);
-      if (isz == 4) scatter_fast_kernel<D, unsigned, true><<<(unsigned)fb, pthreads, (size_t)bytes, s>>>(a, sgn);
-      else scatter_fast_kernel<D, unsigned long long, true><<<(unsigned)fb, pthreads, (size_t)bytes, s>>>(a, sgn);
+      big(isz == 4 ? (const void*)scatter_fast_kernel<D, unsigned, PRIVATE>
+                   : (const void*)scatter_fast_kernel<D, unsigned long long, PRIVATE>);
+      if (isz == 4) scatter_fast_kernel<D, unsigned, PRIVATE><<<(unsigned)fb, pthreads, (size_t)bytes, s>>>(a);
+      else scatter_fast_kernel<D, unsigned long long, PRIVATE><<<(unsigned)fb, pthreads, (size_t)bytes, s>>>(a);
     } else {
+      const bool one = fb <= (long long)sms * 8;
       fb = std::min(fb, (long long)sms * 8);
-      if (isz == 4) scatter_fast_kernel<D, unsigned, false><<<(unsigned)fb, THREADS, 0, s>>>(a, sgn);
-      else scatter_fast_kernel<D, unsigned long long, false><<<(unsigned)fb, THREADS, 0, s>>>(a, sgn);
+      if (one) {
+        if (isz == 4) scatter_fast_kernel<D, unsigned, ONE_TRIP><<<(unsigned)fb, THREADS, 0, s>>>(a);
+        else scatter_fast_kernel<D, unsigned long long, ONE_TRIP><<<(unsigned)fb, THREADS, 0, s>>>(a);
+      } else if (isz == 4) {
+        scatter_fast_kernel<D, unsigned, LOOP><<<(unsigned)fb, THREADS, 0, s>>>(a);
+      } else {
+        scatter_fast_kernel<D, unsigned long long, LOOP><<<(unsigned)fb, THREADS, 0, s>>>(a);
+      }
     }
   } else if (smem) {
     blocks = std::min(blocks, priv_ctas);
