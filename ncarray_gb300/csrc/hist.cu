@@ -255,9 +255,9 @@ struct Sum3 {
 // A block takes 4 * THREADS / CG bins of one tile, four a thread, and splits the
 // tile's pieces over CG groups of threads, merged in a fixed order: with few
 // tiles one has pieces from many CTAs, and a loop over them is a chain of load
-// latency (CG = 4 from 8 pieces a tile on: 64 x 64 bins, 2^20 points 61 -> 44 us
-// a call; 1024 x 1024 bins have 2-3 pieces a tile, CG = 1). The sharing CTAs
-// come from the prefix pass and the weights are sums of three floats (Sum3):
+// latency (CG = 8 from 8 pieces a tile on: 64 x 64 bins, 2^20 weighted points 54
+// us a call with CG = 4, 48 with 8; 1024 x 1024 bins have 2-3 pieces a tile,
+// CG = 1). The sharing CTAs come from the prefix pass and the weights are sums of three floats (Sum3):
 // 64-bit divisions and float64 adds and conversions per bin were most of the
 // pass (50-65 us for 1024 x 1024 weighted bins, 20-22 with pairs of floats;
 // with three a call takes the same time within 1 us). The output's old value is
@@ -271,7 +271,7 @@ tile_combine_kernel(long long nbins, int G, const long long* __restrict__ PV,
                     float* __restrict__ wsum, int ntiles, const int2* __restrict__ ctas) {
   static_assert(TB % (4 * THREADS) == 0, "a block's bins lie in one tile");
   constexpr int Q = THREADS / CG;   // threads per group, four bins each
-  constexpr int LOADS = CG > 1 ? 4 : 1;   // (2 pieces a tile with CG = 1: nothing to batch)
+  constexpr int LOADS = WEIGHTED ? 4 : 8;
   __shared__ int s_bad;
   __shared__ unsigned long long scn[CG > 1 ? CG - 1 : 1][CG > 1 ? Q : 1][4];
   __shared__ Sum3 sw[CG > 1 && WEIGHTED ? CG - 1 : 1][CG > 1 && WEIGHTED ? Q : 1][4];
@@ -460,8 +460,13 @@ extern "C" int32_t nca_hist2d(const float* x, const float* y, const float* w, in
       int per_sm = 0;
       check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, acc_fn, ACC_THREADS, smem), "occupancy");
       if (per_sm < 1) per_sm = 1;
-      // a CTA's records should outnumber the bins it clears and stores
-      const int G = (int)std::max<long long>(1, std::min<long long>((long long)sms * per_sm, n / std::min<long long>(TB, nbins) + 1));
+      // Unweighted, a CTA's records should outnumber the bins it clears and stores
+      // (2^20 points into 100 x 100 bins 38 us, 44 with every CTA). Weighted points
+      // that crowd into few bins are bound by the chains of adds to one address, so
+      // every CTA takes a share of them (2^20 points in one of 128 x 128 bins 241
+      // us, 485 with 65 CTAs; spread evenly 54 either way).
+      const int G = (int)(weighted ? (long long)sms * per_sm
+                                   : std::max<long long>(1, std::min<long long>((long long)sms * per_sm, n / std::min<long long>(TB, nbins) + 1)));
       const long long nslots = (long long)(G + ntiles) * TB;
       const size_t bytes = 4 * 256 + Buckets::bytes(n, ntiles, weighted) + (size_t)nslots * (weighted ? 12 : 4);
       StreamScratch scratch(bytes, s);
@@ -490,8 +495,8 @@ extern "C" int32_t nca_hist2d(const float* x, const float* y, const float* w, in
                                                                        bk.ctas);
       };
       if (G >= 8 * ntiles) {
-        if (weighted) combine(tile_combine_kernel<true, 4>, 4);
-        else combine(tile_combine_kernel<false, 4>, 4);
+        if (weighted) combine(tile_combine_kernel<true, 8>, 8);
+        else combine(tile_combine_kernel<false, 8>, 8);
       } else {
         if (weighted) combine(tile_combine_kernel<true, 1>, 1);
         else combine(tile_combine_kernel<false, 1>, 1);

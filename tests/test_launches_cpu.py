@@ -62,3 +62,20 @@ for points, w in ((7, laplacian7()), (27, laplacian27())):
     for points, shape, three in fake_cuda.run(code, tmp_path):
         want = [False] * 11 if tuple(shape) in flat else [True] * 3 + [False] * 2
         assert three == want, (points, shape)
+
+
+def test_weighted_histogram_uses_every_cta(built_lib, tmp_path):
+    """2^20 weighted points accumulate on one CTA per resident slot even where the bins outnumber a CTA's records: points
+    that crowd into one bin are as many serial adds as a CTA has."""
+    code = """
+from ncarray_gb300.hist import hist2d_into
+fake.fake_resident(1)
+n = 1 << 20
+x, y, w = (array((n,), DType.float32) for _ in range(3))
+result = []
+for nb in (8, 128, 1024):
+    c, s = array((nb, nb), DType.uint64), array((nb, nb), DType.float32)
+    hist2d_into(x, y, c, (0.0, 1.0), (0.0, 1.0), w, s)
+    result.append([k["grid"][0] for k in launches() if "accumulate" in k["launch"]])
+"""
+    assert fake_cuda.run(code, tmp_path) == [[152]] * 3
