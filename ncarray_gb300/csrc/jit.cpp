@@ -1317,7 +1317,10 @@ static void plan_pairs(const Space& s, Spec& sp) {
 // kind 2 on row segments (see the kernel): for rows that keep at least 0.6 of a
 // warp's lanes busy, when a thread gets more than one group: U groups of a row
 // and, when some operands stay put along another dim, F indices of that dim per
-// thread, within about 48 registers of operands and with 32 warps per SM left.
+// thread, within about 48 registers of operands (24 where a group is one 4-byte
+// value: 32 and 48 of them cost the warps that hide their latency, 4 and 6
+// crops of (256, 256, 256) float32 added up 58 -> 63 and 74 -> 98 us; with fewer
+// groups 54 and 75) and with 32 warps per SM left.
 // Measured (us, one group per thread -> segments): (raw - dark) * gain over
 // (96, 512, 1024) uint16 frames 53.8 -> 50.9, over a crop of 500 x 1000 from
 // column 3 76.3 -> 55.7 (82.7 without F), of 509 x 1015 141.6 -> 62.5 (80.3);
@@ -1356,7 +1359,7 @@ static void plan_rows(const Space& s, Spec& sp, int sms) {
   for (int u : {8, 4, 2, 1}) {
     const int64_t nseg = cdiv(gi, 32 * u);
     const double busy = (double)gi / (double)(nseg * 32 * u);
-    if (u > 1 && (u * wr * std::max(1, sp.nops) > 48 || (wr >= 4 && u > 2) || rows * nseg < want)) continue;
+    if (u > 1 && (u * wr * std::max(1, sp.nops) > (wr == 1 ? 24 : 48) || (wr >= 4 && u > 2) || rows * nseg < want)) continue;
     if (busy > best + 0.05) { best = busy; sp.rowu = u; }
   }
   if (best < 0.6) { sp.rowu = 0; sp.loopd = -1; sp.invmask = 0; return; }

@@ -79,3 +79,21 @@ for nb in (8, 128, 1024):
     result.append([k["grid"][0] for k in launches() if "accumulate" in k["launch"]])
 """
     assert fake_cuda.run(code, tmp_path) == [[152]] * 3
+
+
+def test_row_segments_bound_their_registers(built_lib, tmp_path):
+    """Groups per thread of odd rows: 8 up to three operands, fewer with more."""
+    code = """
+result = {}
+for n in (2, 3, 4, 6, 12, 24, 48):
+    xs = [array((256, 256, 259), DType.float32)[:, :, 1:258] for _ in range(n)]
+    e = nca.DevExpr.leaf(xs[0])
+    for x in xs[1:]:
+        e = e + x
+    e.evaluate(out=array((256, 256, 257), DType.float32))
+    (c,) = launches()
+    result[n] = c["consts"]["NCA_ROWU"]
+"""
+    got = {int(n): u for n, u in fake_cuda.run(code, tmp_path).items()}
+    assert all(max(u, 1) * n <= 24 or u <= 1 for n, u in got.items()), got
+    assert got[2] == got[3] == 8 and got[4] == got[6] == 4, got
