@@ -366,7 +366,7 @@ struct Spec {
   // operands that do not move along it
   int rowu = 0, loopd = -1, loopf = 1;
   uint32_t invmask = 0;
-  int k4g = 0;       // row-lane form without a stored value: 1 takes unroll rows' loads together
+  int k4g = 0;       // row-lane form: 1 takes unroll rows' loads together
   int k4r = 0;       // kind 4: row lanes per warp (row-lane form, one reduced dim rd); 0: thread per column group
   int rd = 0;
   int k4p = 0;       // kind 4 row-lane form on a persistent grid (equal contiguous ranges of units)
@@ -2240,16 +2240,46 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
     sp.k4r = R;
     sp.rd = rdim;
     const int64_t nset = cdiv(KG, GPC);
-    // Rows' loads taken together need registers, so fewer CTAs are resident (4
-    // to 5 of 256 threads an SM, 7 to 8 for the plain loop): where the sets of
-    // columns are a few times the SMs and cannot be split to fit, that costs a
-    // second round ((256, 256, 1024) float32 maximum over axis 1, 1024 sets:
-    // 58 us against 48) and the plain loop stays. With at most 4 sets an SM the
-    // loads decide; with 16 or more they do for sums ((200, 777, 333) float32
-    // 50 -> 43), not for extremes, whose plain loop has 8 CTAs an SM
-    // ((128, 1200, 1024) float32 maximum 95 against 103).
+    // Whether a lane's rows are loaded several at a time (k4g: 8, stored float64
+    // 2). Their values are in registers, so it pays while those suffice, with
+    // rows enough to fill the last batch (its missing rows read one again), and
+    // where the fewer CTAs that are resident (4 to 5 of 256 threads an SM, 7 to 8
+    // for the plain loop) do not cost a second round. us, plain -> together:
+    //   operands (stored sum of n float32 arrays, (256, 256, 256) over axis 0):
+    //     n = 3 51 -> 49, 8 205 -> 100, 12 206 -> 149, 24 687 -> 1506 (spills);
+    //     (300, 333, 77) over axis 1, 16 arrays 197 -> 285. float64, 2 rows: 4 201
+    //     -> 149, 6 250 -> 252, 12 634 -> 1024
+    //   rows (float32 over axis 0, 10^6 columns): sum of 5 rows 21 -> 25, 20 28 ->
+    //     27, 31 55 -> 43, 33 39 -> 41, 64 56 -> 55; maximum of (33, 5000) 4.5 ->
+    //     6.4; sum and maximum of few columns gain at any length (0.5 to 0.7)
+    //   sets of 64 column groups: up to 4 an SM the loads decide; between 4 and 16
+    //     the second round ((256, 256, 1024) maximum over axis 1, 1024 sets: 48 ->
+    //     58); from 16 on sums gain ((200, 777, 333) 50 -> 43), extremes do not
+    //     ((128, 1200, 1024) maximum 95 -> 103)
+    //   float64 sums are bound by their pipe: (100, 60000) 20.6 -> 24.9, 4 operands
+    //     of (1024, 4096) 48 -> 58; single arrays of few sets gain ((2000, 5000)
+    //     41 -> 33). 8-bit sums beside extremes by their conversions, once long:
+    //     (20000, 500) 33 -> 40
     const bool fill = tps < 0;
-    sp.k4g = fill && !out && (nset <= 4 * (int64_t)sms || (nset >= 16 * (int64_t)sms && has_sum)) ? 1 : 0;
+    const int64_t m = cdiv(RN, R);   // rows of a lane
+    const bool f64 = arith_dtype(tape.compute_dtype) == NCA_FLOAT64;
+    const bool single = (has_sum ? 1 : 0) + (has_max ? 1 : 0) + (has_min ? 1 : 0) == 1;
+    if (out) {
+      sp.k4g = !fill || (m >= 5 && nops <= (f64 ? 6 : 12)) ? 1 : 0;
+      if (fill && f64 && sp.k4g) sp.unroll = unroll = 2;
+    } else {
+      int widest = 1;
+      for (int k = 0; k < nops; ++k) widest = std::max(widest, dtinfo(s.ops[k].dtype).size);
+      const bool filled = m >= 5 && (m <= 8 || 5 * cdiv(m, 8) * 8 <= 7 * m);
+      const bool few = nset <= 4 * (int64_t)sms, many = nset >= 16 * (int64_t)sms;
+      sp.k4g = fill && nops <= 12 && (few ? filled || !single : many && has_sum && filled) ? 1 : 0;
+      if (f64 && has_sum && single && (nops > 1 || m < 16 || (few && nset > 2 * (int64_t)sms))) sp.k4g = 0;
+      if (widest == 1 && !single && RN >= 4096) sp.k4g = 0;
+      if (sp.k4g && few) {
+        sp.lastcta = lastcta;
+        if (nset > (int64_t)sms * resident_ctas(kernel_for(sp, tape))) sp.k4g = 0;
+      }
+    }
     if (fill) tps = RN <= 256 ? 512 : 1024;
     if (tps == 0) {
       // persistent grid: every resident CTA, units of 4R rows split evenly
@@ -2277,6 +2307,7 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
       if (cbytes) check_cuda(cudaMemsetAsync(p, 0, cbytes, stream), "arrival counters");
       launch(fn, G, w, stream);
       sp.k4r = 0;
+      sp.k4g = 0;
       sp.rd = 0;
       sp.k4p = 0;
       return;
@@ -2288,19 +2319,20 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
       // one CTA more than the others sets the time: among up to twice the
       // splits, the best fill of the last round of CTAs over the SMs, at 4.5 % a
       // split for its merge ((256, 100, 200) 72 -> 64 us, (256, 256, 256) 209
-      // -> 177; (128, 128, 128) keeps 3)
+      // -> 177; (128, 128, 128) keeps 3). With few rows the merge costs more than
+      // that ((64, 60000) doubled, one split 14.8 us, two 18.7)
       auto cost = [&](int64_t k) { return (double)(cdiv(nset * k, sms) * sms) / (double)(nset * k) * (1.0 + 0.045 * (double)k); };
       int64_t best = S;
-      for (int64_t k = S; k <= std::min<int64_t>(2 * S + 2, std::max<int64_t>(1, RN / (8 * R))); ++k)
+      for (int64_t k = S; RN >= 128 && k <= std::min<int64_t>(2 * S + 2, std::max<int64_t>(1, RN / (8 * R))); ++k)
         if (cost(k) < cost(best)) best = k;
       S = best;
     }
     int64_t C = cdiv(RN, S);
     CUfunction fn = nullptr;
-    if (sp.k4g && 2 * nset > (sp.vec == 1 ? 8 : 5) * (int64_t)sms) {
+    if (sp.k4g && !out && 2 * nset > (sp.vec == 1 ? 8 : 5) * (int64_t)sms) {
       S = 1;   // two splits of every set would not be resident together (one element a lane: up to 8 CTAs an SM)
       C = RN;
-    } else if (sp.k4g) {
+    } else if (sp.k4g && !out) {
       // every CTA resident at once: a second round that a few CTAs fill takes as
       // long as the first ((1024, 256, 512) int32 sum, 1024 CTAs where 760 fit:
       // 112 us, 512 CTAs 83). As many splits as fit, in whole trips of
@@ -2483,12 +2515,8 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
     return true;
   }
   // row-lane form: 8 rows in flight per row lane (max over axis 1 of (256, 256,
-  // 1024) 0.77 -> 0.81 of measured); the splits are chosen there: -1
-  // (stored float64 expressions take 2 rows at a time: 8 copies of a tape with
-  // its integer-pipe square root leave the instruction cache, (256, 256, 256)
-  // a*b + sqrt|c| - a/2 252 us against 209)
-  if (rows_ok && !k4r_off())
-    run_k4(out && tape.compute_dtype == NCA_FLOAT64 ? 102 : 108, k4r_persistent() ? 0 : -1, k4r_lastcta());
+  // 1024) 0.77 -> 0.81 of measured); rows together and splits are chosen there: -1
+  if (rows_ok && !k4r_off()) run_k4(108, k4r_persistent() ? 0 : -1, k4r_lastcta());
   else run_k4(4, 1024, 0);
   return true;
 }

@@ -97,3 +97,47 @@ for n in (2, 3, 4, 6, 12, 24, 48):
     got = {int(n): u for n, u in fake_cuda.run(code, tmp_path).items()}
     assert all(max(u, 1) * n <= 24 or u <= 1 for n, u in got.items()), got
     assert got[2] == got[3] == 8 and got[4] == got[6] == 4, got
+
+
+OUTER = """
+def outer(shape, axis, dtype, nops=1, ops=(RedOp.SUM,), stored=False):
+    xs = [array(shape, dtype) for _ in range(nops)]
+    e = nca.DevExpr.leaf(xs[0])
+    for x in xs[1:]:
+        e = e + x
+    kept = [n for d, n in enumerate(shape) if d != axis]
+    out = array(shape, e.expr_dtype) if stored else None
+    from ncarray_gb300.array import _red_out_dtype
+    e.evaluate(out=out, reductions=[(op, axis) for op in ops], red_out=[array(kept, _red_out_dtype(op, e.expr_dtype)) for op in ops])
+    (c,) = [c for c in launches() if "outer" in c["launch"]]
+    return c["consts"]["NCA_K4G"] * c["consts"]["NCA_UNROLL"]   # rows loaded together, 0: one by one
+
+
+"""
+
+
+def test_outer_rows_together_only_where_it_pays(built_lib, tmp_path):
+    """Rows loaded together: not with more operands than the registers hold, nor with rows that leave the last batch
+    nearly empty, nor where fewer resident CTAs cost a second round."""
+    code = OUTER + """
+F, D = DType.float32, DType.float64
+big = (256, 256, 256)
+result = {
+    "stored": [outer(big, 0, F, n, stored=True) for n in (1, 3, 12, 13, 24, 48)],
+    "reduced": [outer((1024, 4096), 0, F, n) for n in (1, 3, 12, 13, 24, 48)],
+    "stored64": [outer(big, 0, D, n, stored=True) for n in (1, 6, 7, 24)],
+    "rows": [outer((n, 1000000), 0, F) for n in (5, 16, 20, 32, 33, 64, 100)],
+    "stored_rows": [outer((n, 100000), 0, F, stored=True) for n in (5, 16, 20, 33)],
+    "two": [outer((n, 5000), 0, F, ops=(RedOp.SUM, RedOp.MAX)) for n in (5, 33)],
+    "sum64": [outer(s, 0, D, n) for s, n in (((2000, 5000), 1), ((2000, 5000), 2), ((100, 60000), 1), ((33, 1000000), 1))],
+}
+"""
+    got = fake_cuda.run(code, tmp_path)
+    # 3 CTAs an SM of the form with the loads together: 456 sets of columns at once
+    got["round"] = fake_cuda.run(OUTER + """
+fake.fake_resident(3)
+result = [outer((1200, 4 * 64 * n), 0, DType.float32) for n in (400, 456, 457, 500)]
+""", tmp_path)
+    assert got == {"stored": [8, 8, 8, 0, 0, 0], "reduced": [8, 8, 8, 0, 0, 0], "stored64": [2, 2, 0, 0],
+                   "rows": [0, 0, 8, 8, 0, 8, 8], "stored_rows": [0, 0, 8, 8], "two": [8, 8], "sum64": [8, 0, 0, 0],
+                   "round": [8, 8, 0, 0]}
