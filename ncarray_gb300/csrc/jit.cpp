@@ -1327,13 +1327,14 @@ static void plan_pairs(const Space& s, Spec& sp) {
 // (65536, 1000) bfloat16 times a row 67.7 -> 63.9 (70.4 without F); x * r + c
 // over (4096, 4096) float32 24.8 -> 22.2, over 4001 x 4001 44.3 -> 23.9. Groups
 // of 16 bytes: two per thread (three and more 2-5 % slower). float64 vectors
-// stay on one group per thread: their arithmetic, not the loads, is the longer
-// part, and batching the loads ends its overlap ((256, 256, 256) times a
-// broadcast plane 45.3 against 47.6).
+// and float64 over three operands and more stay on one group per thread: their
+// arithmetic, not the loads, is the longer part, and batching the loads ends its
+// overlap ((256, 256, 256) times a broadcast plane 45.3 against 47.6; x * r + y
+// over odd rows of (96, 509, 1015) 214 against 232).
 static void plan_rows(const Space& s, Spec& sp, int sms) {
   const int ax = s.nd - 1;
   sp.rowu = 0; sp.loopd = -1; sp.loopf = 1; sp.invmask = 0;
-  if (!sp.idx32 || s.out.st[ax] != dtinfo(s.out.dtype).size || (sp.w == NCA_FLOAT64 && sp.vec > 1)) return;
+  if (!sp.idx32 || s.out.st[ax] != dtinfo(s.out.dtype).size || (sp.w == NCA_FLOAT64 && (sp.vec > 1 || sp.nops > 2))) return;
   for (int k = 0; k < sp.nops; ++k) if (s.ops[k].ptr && s.ops[k].pts[ax] != 0) return;
   const int64_t gi = s.shape[ax] / sp.vec, rows = s.total() / std::max<int64_t>(s.shape[ax], 1);
   const int wr = std::max(1, dtinfo(sp.w).size / 4) * sp.vec;   // registers of a loaded group
@@ -1869,10 +1870,16 @@ void expr_eval(const Tape& tape, const nca_view* ops, int nops, const nca_view& 
   bool flat = s.nd == 1 && s.out.st[0] == dtinfo(out.dtype).size && sp.ptrmask == 0;
   for (int k = 0; k < nops && flat; ++k)
     if (s.ops[k].st[0] != 0 && s.ops[k].st[0] != dtinfo(ops[k].dtype).size) flat = false;
-  plan_vec(s, sp, 16, true, flat);
+  // an extent that is no multiple of the vector keeps it where loads decide. 8-byte
+  // arithmetic goes one element per thread: float64 always (x * y + x over 2^24 + 1
+  // elements 72.8 us against 80.3), integers while short (10^6 + 3 int8 4.5 against
+  // 6.3; 2^24 + 1 35.9 against 33.0)
+  const int64_t n1 = s.shape[s.nd - 1];
+  const bool tail = flat && (dtinfo(sp.w).size <= 4 || (sp.w != NCA_FLOAT64 && n1 >= (1 << 22)));
+  plan_vec(s, sp, 16, true, tail);
   if (flat) {
     for (int k = 0; k < nops; ++k) if (sp.op_modes[k] == M_STRIDED && sp.vec > 1) flat = false;
-    if (!flat) plan_vec(s, sp, 16, true);
+    if (!flat && tail) plan_vec(s, sp, 16, true);
   }
   sp.kind = flat ? 1 : 2;
   if (sp.kind == 2) {

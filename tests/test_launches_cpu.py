@@ -141,3 +141,29 @@ result = [outer((1200, 4 * 64 * n), 0, DType.float32) for n in (400, 456, 457, 5
     assert got == {"stored": [8, 8, 8, 0, 0, 0], "reduced": [8, 8, 8, 0, 0, 0], "stored64": [2, 2, 0, 0],
                    "rows": [0, 0, 8, 8, 0, 8, 8], "stored_rows": [0, 0, 8, 8], "two": [8, 8], "sum64": [8, 0, 0, 0],
                    "round": [8, 8, 0, 0]}
+
+
+def test_odd_vectors_and_rows_of_8_byte_arithmetic(built_lib, tmp_path):
+    """Odd 1-D extents keep 16-byte vectors, except float64 and short 8-byte integer arithmetic; float64 rows of three
+    operands take no segments."""
+    code = """
+def flat(n, dtype):
+    x, y = array((n,), dtype), array((n,), dtype)
+    e = nca.DevExpr.leaf(x) + nca.DevExpr.leaf(y)
+    e.evaluate(out=array((n,), e.expr_dtype))
+    (c,) = launches()
+    return c["consts"]["NCA_VEC"]
+
+def rows(nops, dtype):
+    xs = [array((96, 509, 250), dtype)[:, :, 1:250] for _ in range(nops)]
+    e = nca.DevExpr.leaf(xs[0])
+    for x in xs[1:]:
+        e = e + x
+    e.evaluate(out=array((96, 509, 249), e.expr_dtype))
+    (c,) = launches()
+    return c["consts"]["NCA_ROWU"]
+
+F, D, I8 = DType.float32, DType.float64, DType.int8
+result = [[flat(n, t) for n in (1003, (1 << 23) + 1, 1 << 23)] for t in (F, D, I8)] + [[rows(n, t) for n in (2, 3)] for t in (F, D)]
+"""
+    assert fake_cuda.run(code, tmp_path) == [[4, 4, 4], [1, 1, 2], [1, 2, 2], [8, 8], [8, 0]]
