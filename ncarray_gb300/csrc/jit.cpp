@@ -1946,6 +1946,7 @@ void expr_eval(const Tape& tape, const nca_view* ops, int nops, const nca_view& 
                     std::to_string(tape.compute_dtype) + "|";
   for (int k = 0; k < nops; ++k) key += std::to_string(ops[k].dtype) + ".";
   key += "|v" + std::to_string(sp.vec) + "|n" + size_class(total) + "|d" + std::to_string(s.nd);
+  if (sp.rowu > 0) key += "|s";   // row segments: another kernel than the one the plain key's choices were made for
   auto run = [&](const std::vector<int>& c) {
     Spec sc = sp;
     sc.block = c[0];
@@ -2488,18 +2489,25 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
     sp.rd = 0;
     sp.k4b = 0;
   }
+  // untuned: the row-lane form with 8 rows in flight per row lane (max over axis 1
+  // of (256, 256, 1024) 0.77 -> 0.81 of measured), which chooses rows together and
+  // splits itself (-1); else 4 rows per thread and 1024 threads per SM
+  const std::vector<int> untuned = rows_ok && !k4r_off() ? std::vector<int>{108, k4r_persistent() ? 0 : -1, k4r_lastcta()}
+                                                         : std::vector<int>{4, 1024, 0};
   // schedule: the autotuner's cached choice for this (dtypes, ops, stored
-  // value, kept and reduced size class, dims), else 4 rows in flight and 1024
-  // threads per SM; searched (rows 4 / 8, 512 / 1024 / 2048 threads per SM)
-  // when the kernel writes nothing it reads
-  std::string key = "red|k4|" + std::to_string(tape.compute_dtype) + "|" + std::to_string(red_ops) + "|o" +
+  // value, kept and reduced size class, dims), else the untuned one; searched
+  // (the untuned one first, rows 4 / 8, 512 / 1024 / 2048 threads per SM) when the
+  // kernel writes nothing it reads. The key's "k4b": choices stored under "k4"
+  // were made without the present untuned form among them and would undo it
+  std::string key = "red|k4b|" + std::to_string(tape.compute_dtype) + "|" + std::to_string(red_ops) + "|o" +
                     std::to_string(out ? out->dtype : -1) + "|";
   for (int k = 0; k < nops; ++k) key += std::to_string(ops[k].dtype) + ".";
   key += "|r" + size_class(RN) + "|k" + size_class(KN) + "|d" + std::to_string(s.nd) + "|v" + std::to_string(sp.vec);
   std::vector<int> choice;
   if (tune_get(key, choice) && choice.size() == 3 &&
       (choice[0] == 4 || choice[0] == 8 || (rows_ok && (choice[0] == 102 || choice[0] == 104 || choice[0] == 108))) &&
-      (choice[1] == 512 || choice[1] == 1024 || choice[1] == 2048 || (choice[0] >= 100 && choice[1] == 0)) &&
+      (choice[1] == 512 || choice[1] == 1024 || choice[1] == 2048 || (choice[0] >= 100 && choice[1] == 0) ||
+       (choice[0] == 108 && choice[1] == -1)) &&
       (choice[2] == 0 || choice[2] == 1)) {
     run_k4(choice[0], choice[1], choice[2]);
     return true;
@@ -2508,8 +2516,10 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
   for (int k = 0; k < nred; ++k) routs.push_back(rv[(size_t)k].out);
   if (out) routs.push_back(*out);
   if (KN * RN >= (1 << 16) && tune_should_search(stream) && rerun_safe(ops, nops, routs.data(), (int)routs.size())) {
-    std::vector<std::vector<int>> cands = {{4, 1024, 0}, {8, 1024, 0}, {4, 2048, 0}, {8, 2048, 0}, {8, 512, 0},
-                                           {4, 1024, 1}, {8, 512, 1}};
+    std::vector<std::vector<int>> cands = {untuned};
+    for (auto c : std::vector<std::vector<int>>{{4, 1024, 0}, {8, 1024, 0}, {4, 2048, 0}, {8, 2048, 0}, {8, 512, 0},
+                                                {4, 1024, 1}, {8, 512, 1}})
+      if (c != untuned) cands.push_back(c);
     if (rows_ok)
       for (auto c : std::vector<std::vector<int>>{{104, 0, 0}, {104, 2048, 1}, {104, 2048, 0}, {102, 2048, 1}, {104, 1024, 1},
                                                   {108, 1024, 1}, {108, 512, 1}, {104, 512, 1}})
@@ -2521,10 +2531,7 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
     run_k4(cands[(size_t)best][0], cands[(size_t)best][1], cands[(size_t)best][2]);
     return true;
   }
-  // row-lane form: 8 rows in flight per row lane (max over axis 1 of (256, 256,
-  // 1024) 0.77 -> 0.81 of measured); rows together and splits are chosen there: -1
-  if (rows_ok && !k4r_off()) run_k4(108, k4r_persistent() ? 0 : -1, k4r_lastcta());
-  else run_k4(4, 1024, 0);
+  run_k4(untuned[0], untuned[1], untuned[2]);
   return true;
 }
 

@@ -74,11 +74,12 @@ def build() -> Path:
     return out
 
 
-def run(code: str, cache_dir, **env):
-    """The child's `result`; a child that dies raises with its status."""
+def run(code: str, cache_dir, args=(), **env):
+    """The child's `result`; a child that dies raises with its status. `args` follow the library in sys.argv."""
+    Path(cache_dir).mkdir(exist_ok=True)
     env = dict(os.environ, NCA_GB300_CACHE_DIR=str(cache_dir),
                PYTHONPATH=str(ROOT) + os.pathsep + os.environ.get("PYTHONPATH", ""), **env)
-    r = subprocess.run([sys.executable, "-c", PRELUDE + code + "\nprint(json.dumps(result))", str(build())], env=env, cwd=ROOT,
+    r = subprocess.run([sys.executable, "-c", PRELUDE + code + "\nprint(json.dumps(result))", str(build()), *map(str, args)], env=env, cwd=ROOT,
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, f"child ended with {r.returncode}\n{r.stderr[-3000:]}"
     return json.loads(r.stdout.strip().splitlines()[-1])

@@ -167,3 +167,33 @@ F, D, I8 = DType.float32, DType.float64, DType.int8
 result = [[flat(n, t) for n in (1003, (1 << 23) + 1, 1 << 23)] for t in (F, D, I8)] + [[rows(n, t) for n in (2, 3)] for t in (F, D)]
 """
     assert fake_cuda.run(code, tmp_path) == [[4, 4, 4], [1, 1, 2], [1, 2, 2], [8, 8], [8, 0]]
+
+
+REDUCE = """
+x = array((4096, 16384), DType.float32)
+out = array((16384,), DType.float32)
+
+def launch():
+    nca.DevExpr.leaf(x).evaluate(reductions=[(RedOp.SUM, 0)], red_out=[out])
+    return launches()
+
+"""
+
+
+def test_tuner_knows_the_untuned_outer_reduction(built_lib, tmp_path):
+    """A search includes the form that runs untuned and its stored choice is read back; choices of the former key, made
+    without it, are not."""
+    plain = fake_cuda.run(REDUCE + "result = launch()", tmp_path / "a")
+    # every candidate takes the same (fake) time: the first one, the untuned form, is stored
+    found = fake_cuda.run(REDUCE + "tune.set_mode(2)\nls = launch()\nresult = [ls, tune.entries(sys.argv[2])]", tmp_path / "b",
+                          args=[tmp_path / "b"])
+    assert plain[0] in found[0] and found[0][-1] == plain[0]
+    (key, value), = found[1].items()
+    assert value == [108, -1, 1]
+    assert fake_cuda.run(REDUCE + "result = launch()", tmp_path / "b") == plain
+    old = tmp_path / "c"
+    old.mkdir()
+    (old / "tune.txt").write_text(key.replace("red|k4b|", "red|k4|") + " 8 512 0\n")
+    assert fake_cuda.run(REDUCE + "result = launch()", old) == plain
+    (old / "tune.txt").write_text(key + " 8 512 0\n")
+    assert fake_cuda.run(REDUCE + "result = launch()", old) != plain
