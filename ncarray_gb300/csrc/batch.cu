@@ -48,7 +48,7 @@ struct nca_batch {
   void* d_status = nullptr;   // int: NCA_ERR_TIMEOUT after a wait that ran out
   long long nchunks = 0;
   // schedule
-  long long chunk_bytes = 256 * 1024;
+  long long total_bytes = 0, chunk_bytes = 256 * 1024;
   int threads = 256, slab = 16384, ctas_per_sm = 3;
   std::string shape_class;
   // graph
@@ -536,7 +536,8 @@ std::string shape_class(const nca_batch* B) {
   const int ln = B->n > 0 ? (int)std::log2((double)B->n) : 0;
   const int mix = B->n > 0 ? (int)(4.0 * n16 / B->n + 0.5) : 0;
   std::ostringstream os;
-  os << "batch_b" << lb << "_n" << ln << "_m" << mix;
+  // ("batch2": choices stored under "batch" were timed with the chunks in array order)
+  os << "batch2_b" << lb << "_n" << ln << "_m" << mix;
   return os.str();
 }
 
@@ -595,6 +596,7 @@ int32_t nca_batch_create(const nca_batch_item* items, int32_t n_items, nca_batch
       B->shape_class = shape_class(B);
       long long total = 0;
       for (const auto& it : B->items) total += it.length * (it.dtype == NCA_FLOAT32 ? 4 : 2);
+      B->total_bytes = total;
       B->chunk_bytes = chunk_bytes_for(total, (long long)sm_count(B->dev) * B->ctas_per_sm, B->slab);
       load_tuned(B);
       // NCA_BATCH_SCHEDULE="<chunk bytes>,<threads>,<slab bytes>,<CTAs per SM>" overrides the tuned schedule
@@ -682,6 +684,10 @@ int32_t nca_batch_autotune(nca_batch* B, nca_batch_result* results, void* stream
     check_cuda(cudaFuncSetAttribute(batch_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     NSLAB * 32768 + 16 * NSLAB),
                "batch smem");
+    // the untuned schedule first (chunks of a CTA's share), then fixed chunk sizes
+    const nca_batch plain;
+    cands.push_back({chunk_bytes_for(B->total_bytes, (long long)sm_count(B->dev) * plain.ctas_per_sm, plain.slab), plain.threads,
+                     plain.slab, plain.ctas_per_sm});
     for (long long cb : {256ll << 10, 512ll << 10, 1024ll << 10})
       for (int sl : {8192, 16384, 32768})
         for (int cps : {2, 3, 4}) {
@@ -691,7 +697,6 @@ int32_t nca_batch_autotune(nca_batch* B, nca_batch_result* results, void* stream
                      "occupancy");
           if (schedule_ok(cb, 256, sl, cps) && resident >= cps) cands.push_back({cb, 256, sl, cps});
         }
-    if (cands.empty()) cands.push_back({256ll << 10, 256, 16384, 3});
     cudaEvent_t e0, e1;
     check_cuda(cudaEventCreate(&e0), "event");
     check_cuda(cudaEventCreate(&e1), "event");

@@ -197,3 +197,44 @@ def test_tuner_knows_the_untuned_outer_reduction(built_lib, tmp_path):
     assert fake_cuda.run(REDUCE + "result = launch()", old) == plain
     (old / "tune.txt").write_text(key + " 8 512 0\n")
     assert fake_cuda.run(REDUCE + "result = launch()", old) != plain
+
+
+BATCH = """
+lengths = [1000 + 2000 * k for k in range(160)]
+items = (_lib.BatchItem * len(lengths))()
+for it, n in zip(items, lengths):
+    it.data, it.length, it.dtype = 1 << 40, n, int(DType.float32)
+
+def create():
+    h = ctypes.c_void_p()
+    _lib.call("nca_batch_create", items, len(lengths), ctypes.byref(h), None)
+    return h
+
+def schedule(h):
+    c, t, u, n = ctypes.c_int64(), ctypes.c_int32(), ctypes.c_int32(), ctypes.c_int32()
+    _lib.call("nca_batch_schedule", h, ctypes.byref(c), ctypes.byref(t), ctypes.byref(u), ctypes.byref(n))
+    return [c.value, t.value, u.value, n.value]
+
+"""
+
+
+def test_batch_tuner_knows_the_untuned_schedule(built_lib, tmp_path):
+    """autotune() times the untuned schedule too (the first of equal candidates is kept); schedules stored before the
+    chunks were ordered are not read back."""
+    plain = fake_cuda.run(BATCH + "result = schedule(create())", tmp_path / "a")
+    assert plain[0] % 16384 == 0 and 128 * 1024 <= plain[0] <= 512 * 1024 and plain[0] not in (256 << 10, 512 << 10)
+    code = """
+h = create()
+_lib.call("nca_batch_autotune", h, ctypes.c_void_p(1 << 41), None)
+result = [schedule(h), open(sys.argv[2] + "/batch_tune_ws.txt").read()]
+"""
+    got, text = fake_cuda.run(BATCH + code, tmp_path / "b", args=[tmp_path / "b"])
+    assert got == plain
+    key, *value = text.split()
+    assert fake_cuda.run(BATCH + "result = schedule(create())", tmp_path / "b") == plain
+    old = tmp_path / "c"
+    old.mkdir()
+    (old / "batch_tune_ws.txt").write_text(f"{key.replace('batch2_', 'batch_')} {1 << 20} 256 8192 2\n")
+    assert fake_cuda.run(BATCH + "result = schedule(create())", old) == plain
+    (old / "batch_tune_ws.txt").write_text(f"{key} {1 << 20} 256 8192 2\n")
+    assert fake_cuda.run(BATCH + "result = schedule(create())", old) != plain
