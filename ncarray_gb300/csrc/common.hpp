@@ -109,10 +109,11 @@ struct StreamScratch {
 
 // `n` arrival counters, all zero, for a kernel on stream `s` that leaves them
 // zero; null where the caller has to zero counters of its own. The marked ones
-// are for kernels that may leave any count: launch_mark() in the high half.
+// are for kernels that may leave any count: the launch's mark in the upper 44
+// bits, a count of up to 2^20 - 1 arrivals (a kernel's CTAs) in the lower 20.
 uint32_t* arrival_counters(int64_t n, cudaStream_t s);
 unsigned long long* marked_counters(int64_t n, cudaStream_t s);
-uint32_t launch_mark();
+uint64_t launch_mark();
 
 // ---- chunk tables of the batched kernels --------------------------------------
 // Bytes per chunk: a CTA's share of the batch in whole slabs, between 128 and

@@ -807,7 +807,8 @@ int* jit_status_word() {
 //
 // Kernels with bounded waits may stop early and leave any count behind, so
 // they take marked words instead: 64 bits, the launch's mark above the count,
-// and a word with another mark counts from zero.
+// and a word with another mark counts from zero. (A mark comes again after 2^44
+// launches.)
 static void* stream_words(bool marked, int64_t n, cudaStream_t stream) {
   static std::mutex mu;
   struct Dev { void *plain = nullptr, *marked = nullptr; std::unordered_map<unsigned long long, int> slot; };
@@ -843,10 +844,9 @@ uint32_t* arrival_counters(int64_t n, cudaStream_t stream) {
 unsigned long long* marked_counters(int64_t n, cudaStream_t stream) {
   return static_cast<unsigned long long*>(stream_words(true, n, stream));
 }
-uint32_t launch_mark() {
-  static std::atomic<uint32_t> next{1};
-  uint32_t m = next++;
-  return m ? m : next++;   // 0 is what a cleared word holds
+uint64_t launch_mark() {
+  static std::atomic<uint64_t> next{1};   // 0 is what a cleared word holds
+  return next++ << 20;
 }
 
 // reads and clears the stencil status word (synchronises the stream)

@@ -19,6 +19,7 @@
 namespace {
 struct Kernel {
   std::string name, defines;   // JSON members of the NCA_ constants
+  int chunk_word = -1;         // of a generated kernel: which argument word is its chunk
 };
 std::mutex mu;
 std::string log_text;
@@ -32,10 +33,10 @@ void record(const std::string& line) {
   std::lock_guard<std::mutex> lk(mu);
   log_text += line + "\n";
 }
-void record_launch(const Kernel* k, dim3 g, dim3 b, size_t smem) {
+void record_launch(const Kernel* k, dim3 g, dim3 b, size_t smem, const unsigned long long* words = nullptr) {
   record("{\"launch\": \"" + k->name + "\", \"grid\": [" + std::to_string(g.x) + ", " + std::to_string(g.y) + ", " +
          std::to_string(g.z) + "], \"block\": " + std::to_string(b.x) + ", \"smem\": " + std::to_string(smem) +
-         ", \"consts\": {" + k->defines + "}}");
+         (words && k->chunk_word >= 0 ? ", \"chunk\": " + std::to_string(words[k->chunk_word]) : "") + ", \"consts\": {" + k->defines + "}}");
 }
 // "#define NCA_NAME <integer>" lines of a source as JSON members
 std::string constants(const char* src) {
@@ -61,12 +62,15 @@ CUresult module_load(CUmodule* m, const void* image) {
   return CUDA_SUCCESS;
 }
 CUresult module_function(CUfunction* f, CUmodule m, const char* name) {
-  *f = (CUfunction) new Kernel{name, constants(((std::string*)m)->c_str())};
+  auto* k = new Kernel{name, constants(((std::string*)m)->c_str())};
+  const size_t at = k->defines.find("\"NCA_W_CHUNK\": ");
+  if (at != std::string::npos) k->chunk_word = atoi(k->defines.c_str() + at + 15);
+  *f = (CUfunction)k;
   return CUDA_SUCCESS;
 }
 CUresult launch(CUfunction f, unsigned gx, unsigned gy, unsigned gz, unsigned bx, unsigned by, unsigned bz, unsigned smem,
-                CUstream, void**, void**) {
-  record_launch((const Kernel*)f, dim3(gx, gy, gz), dim3(bx, by, bz), smem);
+                CUstream, void** args, void**) {
+  record_launch((const Kernel*)f, dim3(gx, gy, gz), dim3(bx, by, bz), smem, (const unsigned long long*)args[0]);
   return CUDA_SUCCESS;
 }
 CUresult func_attribute(CUfunction, CUfunction_attribute, int) { return CUDA_SUCCESS; }
@@ -106,7 +110,7 @@ API void __cudaUnregisterFatBinary(void**) {}
 API void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
 API void __cudaRegisterFunction(void**, const char* host, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*, int*) {
   std::lock_guard<std::mutex> lk(mu);
-  runtime_kernels[host] = new Kernel{name, ""};
+  runtime_kernels[host] = new Kernel{name, "", -1};
 }
 API unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t smem, cudaStream_t s) {
   call_grid = g; call_block = b; call_smem = smem; call_stream = s;

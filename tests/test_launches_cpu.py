@@ -238,3 +238,21 @@ result = [schedule(h), open(sys.argv[2] + "/batch_tune_ws.txt").read()]
     assert fake_cuda.run(BATCH + "result = schedule(create())", old) == plain
     (old / "batch_tune_ws.txt").write_text(f"{key} {1 << 20} 256 8192 2\n")
     assert fake_cuda.run(BATCH + "result = schedule(create())", old) != plain
+
+
+def test_launch_marks_leave_the_count_its_bits(built_lib, tmp_path):
+    """The marks of staged reductions' counters: another one for each launch, above 20 bits of count, so that one comes
+    again after 2^44 launches instead of 2^32."""
+    code = """
+t = array((64, 64, 128, 8), DType.int32).transpose(3, 1, 2, 0)
+e = nca.DevExpr.leaf(t) * np.int32(3)
+kept = [t.shape[d] for d in (0, 1, 3)]
+out, red = array(t.shape, e.expr_dtype), array(kept, e.expr_dtype)
+for _ in range(3):
+    e.evaluate(out, [(RedOp.MAX, 2)], [red])
+result = [[c["consts"]["NCA_KIND"], c["chunk"]] for c in launches()]
+"""
+    got = fake_cuda.run(code, tmp_path)
+    assert [k for k, _ in got] == [7] * 3
+    marks = [m for _, m in got]
+    assert all(m and m % 2**20 == 0 for m in marks) and len(set(marks)) == 3
