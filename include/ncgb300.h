@@ -156,6 +156,9 @@ int32_t nca_jit_set_cache_dir(const char* dir);
  * NVRTC for `arch` (e.g. "sm_103a") without touching a device. No reference
  * counterpart (the reference only compiles on first use, rtcompiler.cc:445-510). */
 int32_t nca_jit_selftest(const char* arch, int32_t* n_compiled);
+/* The same for the forms that a class takes by shape and operand count (row
+ * segments, outer reductions with several rows' loads together). */
+int32_t nca_jit_selftest_forms(const char* arch, int32_t* n_compiled);
 
 /* ---- launch-schedule autotuner ------------------------------------------- */
 /* Schedules (stencil tile shape and z-march depth; threads per block, vector

@@ -90,6 +90,7 @@ EXPORTS = {
     "nca_jit_stats": (c_int32, [POINTER(c_int64), POINTER(c_int64), POINTER(c_int64)]),
     "nca_jit_set_cache_dir": (c_int32, [c_char_p]),
     "nca_jit_selftest": (c_int32, [c_char_p, POINTER(c_int32)]),
+    "nca_jit_selftest_forms": (c_int32, [c_char_p, POINTER(c_int32)]),
     "nca_expr_eval": (c_int32, [POINTER(Tape), POINTER(View), c_int32, POINTER(View), c_void_p]),
     "nca_expr_reduce": (c_int32, [POINTER(Tape), POINTER(View), c_int32, POINTER(View), POINTER(Reduction), c_int32, c_void_p]),
     "nca_expr_multi": (c_int32, [POINTER(Tape), c_int32, POINTER(View), c_int32, POINTER(View), POINTER(Reduction),

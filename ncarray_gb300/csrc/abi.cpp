@@ -49,6 +49,14 @@ int32_t nca_jit_selftest(const char* arch, int32_t* n_compiled) {
   });
 }
 
+// The same for the forms chosen by shape and operand count inside a class.
+int32_t nca_jit_selftest_forms(const char* arch, int32_t* n_compiled) {
+  return guarded([&] {
+    const int n = jit_selftest_forms(arch);
+    if (n_compiled) *n_compiled = n;
+  });
+}
+
 int32_t nca_expr_eval(const nca_tape* tape, const nca_view* operands, int32_t n_operands,
                       const nca_view* out, void* stream) {
   return guarded([&] {

@@ -2729,24 +2729,55 @@ int jit_selftest(const char* arch) {
     nvrtc_compile(gen_source(sp, t), a);
     ++n;
   }
-  // kind 2 on row segments: plain, with a hoisting loop dim (operand 0 stays put along it), pointer operand.
-  // Compiled but not counted: the count that nca_jit_selftest reports is known to its callers.
-  for (int di : {1, 3}) {
-    auto& d = dts[di];
+  n += batch_expr_selftest(a.c_str());
+  n += stencil_tile_selftest(a.c_str());
+  return n;
+}
+
+// The same for the forms that the planner chooses by shape and operand count
+// inside those classes: row segments (kind 2) and rows taken together (kind 4).
+int jit_selftest_forms(const char* arch) {
+  const std::string a = arch ? arch : "sm_103a";
+  int n = 0;
+  auto compile = [&](const Spec& sp, const Tape& t) {
+    nvrtc_compile(gen_source(sp, t), a);
+    ++n;
+  };
+  Tape t;
+  auto I = [](int op, int idx) { return (uint32_t)(op << 24) | (uint32_t)idx; };
+  t.instrs = {I(NCA_OP_LOAD_NCARR, 0), I(NCA_OP_LOAD_CONST, 0), I(NCA_OP_MUL, 0), I(NCA_OP_LOAD_NCARR, 1), I(NCA_OP_ADD, 0),
+              I(NCA_OP_LOAD_NCARR, 2), I(NCA_OP_ADD, 0)};
+  t.scalar_dtypes = {NCA_FLOAT64};
+  double half = 0.5;
+  uint64_t hb;
+  memcpy(&hb, &half, 8);
+  t.scalar_slots = {hb};
+  t.n_arrays = 3;
+  const int dts[][4] = {{NCA_FLOAT32, NCA_FLOAT32, NCA_INT32, 4}, {NCA_FLOAT32, NCA_BFLOAT16, NCA_BFLOAT16, 4}};   // w, out/r, op dtype, vec
+  for (auto& d : dts) {
+    t.compute_dtype = d[0];
+    t.result_dtype = d[1];
+    // row segments: plain, with a hoisting loop dim (operand 0 stays put along it), pointer operand
     Spec sp;
     sp.kind = 2; sp.nops = 3; sp.nd = 3; sp.vec = 1; sp.idx32 = 1; sp.w = d[0]; sp.r = d[1]; sp.out_dtype = d[1]; sp.nscal = 1;
     sp.has_out = true;
-    t.compute_dtype = d[0]; t.result_dtype = d[1];
     sp.op_dtypes = {d[2], d[2], d[2]}; sp.op_modes = {M_CONTIG, M_CONST, M_CONTIG}; sp.op_salias = {-1, -1, -1};
     sp.rowu = 4;
-    nvrtc_compile(gen_source(sp, t), a);
+    compile(sp, t);
     sp.loopd = 0; sp.loopf = 4; sp.invmask = 1u;
-    nvrtc_compile(gen_source(sp, t), a);
+    compile(sp, t);
     sp.loopd = -1; sp.loopf = 1; sp.invmask = 0; sp.ptrmask = 4u; sp.vec = std::min(d[3], 4); sp.op_modes[2] = M_STRIDED;
-    nvrtc_compile(gen_source(sp, t), a);
+    compile(sp, t);
+    // rows together, with and without a stored value
+    Spec s4;
+    s4.kind = 4; s4.nops = 3; s4.nd = 3; s4.vec = d[3]; s4.idx32 = 1; s4.w = d[0]; s4.r = d[1]; s4.out_dtype = d[1]; s4.nscal = 1;
+    s4.op_dtypes = {d[2], d[2], d[2]}; s4.op_modes = {M_CONTIG, M_CONST, M_STRIDED};
+    s4.nred = 2; s4.red_ops = 0u | (2u << 4); s4.has_sum = s4.has_max = true; s4.kept_mask = 1u | 4u;
+    s4.k4r = 4; s4.rd = 1; s4.lastcta = 1; s4.k4g = 1; s4.unroll = 8;
+    compile(s4, t);
+    s4.has_out = true; s4.unroll = 2;
+    compile(s4, t);
   }
-  n += batch_expr_selftest(a.c_str());
-  n += stencil_tile_selftest(a.c_str());
   return n;
 }
 

@@ -80,6 +80,7 @@ std::string jit_storage_uint(int size);
 
 namespace nca {
 int jit_selftest(const char* arch);
+int jit_selftest_forms(const char* arch);
 // NVRTC compile of `source` for `arch` without loading it (fails on errors)
 void jit_compile_only(const std::string& source, const std::string& arch);
 int batch_expr_selftest(const char* arch);

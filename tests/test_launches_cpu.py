@@ -1,6 +1,9 @@
 """What the host side of a call launches, without a GPU (tests/fake_cuda)."""
+import ctypes
+
 import pytest
 
+from ncarray_gb300 import _lib
 from tests import fake_cuda
 
 
@@ -256,3 +259,20 @@ result = [[c["consts"]["NCA_KIND"], c["chunk"]] for c in launches()]
     assert [k for k, _ in got] == [7] * 3
     marks = [m for _, m in got]
     assert all(m and m % 2**20 == 0 for m in marks) and len(set(marks)) == 3
+
+
+@pytest.mark.parametrize("name", ["nca_jit_selftest", "nca_jit_selftest_forms"])
+def test_selftests_report_what_they_compile(built_lib, tmp_path, name):
+    code = f"""
+n = ctypes.c_int32()
+_lib.call("{name}", b"sm_103a", ctypes.byref(n))
+result = [n.value, sum("compile" in c for c in calls())]
+"""
+    reported, compiled = fake_cuda.run(code, tmp_path)
+    assert reported == compiled > 0
+
+
+def test_nvrtc_compiles_every_form(built_lib):
+    n = ctypes.c_int32(0)
+    _lib.call("nca_jit_selftest_forms", b"sm_103a", ctypes.byref(n))
+    assert n.value == 10
