@@ -9,11 +9,11 @@
 //      global atomics;
 //   3. the caller accumulates record ranges tile by tile in shared memory and
 //      combines the pieces.
-// A source says what an element is (all arrays are 4-byte elements):
-//   NA           arrays read per element: the key arrays, then the value
-//   VAL          records carry the last array's word
+// The points as their source (all arrays are 4-byte elements):
+//   VAL          records carry a weight
+//   NA           arrays read per element: x, y and the weight
 //   array(k)     base of array k
-//   bin(a, b)    bin of key words a (array 0) and b (array 1), or NO_BIN
+//   bin(a, b)    bin of the words a of x and b of y, or NO_BIN
 //   direct(bin, word)  adds a record with global atomics
 #pragma once
 #include <cstdint>
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256) tile_sample_kernel(Src src, long long n, 
       const long long i = s * SAMPLE * 1024 + k * 256 + threadIdx.x;
       const long long j = i < n ? i : n - 1;
       a[k] = __ldg(src.array(0) + j);
-      b[k] = Src::NA - (Src::VAL ? 1 : 0) > 1 ? __ldg(src.array(1) + j) : 0u;
+      b[k] = __ldg(src.array(1) + j);
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(ST, Src::VAL ? 2 : 3)
 tile_scatter_kernel(Src src, long long n, int ntiles, const long long* __restrict__ off, const long long* __restrict__ cap,
                     unsigned long long* __restrict__ fill, unsigned short* __restrict__ rec_bin,
                     unsigned* __restrict__ rec_val, int* __restrict__ status) {
-  constexpr int NA = Src::NA, NK = NA - (Src::VAL ? 1 : 0);
+  constexpr int NA = Src::NA;
   constexpr uint32_t ABYTES = CHUNK * 4;
   extern __shared__ __align__(128) unsigned char sm[];
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
@@ -207,15 +207,15 @@ tile_scatter_kernel(Src src, long long n, int ntiles, const long long* __restric
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         a[h] = buf[h * ST + tid];
-        if (NK > 1) b[h] = buf[CHUNK / 4 + h * ST + tid];
-        if (Src::VAL) v[h] = buf[NK * (CHUNK / 4) + h * ST + tid];
+        b[h] = buf[CHUNK / 4 + h * ST + tid];
+        if (Src::VAL) v[h] = buf[2 * (CHUNK / 4) + h * ST + tid];
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        bins[4 * h] = src.bin(a[h].x, NK > 1 ? b[h].x : 0u);
-        bins[4 * h + 1] = src.bin(a[h].y, NK > 1 ? b[h].y : 0u);
-        bins[4 * h + 2] = src.bin(a[h].z, NK > 1 ? b[h].z : 0u);
-        bins[4 * h + 3] = src.bin(a[h].w, NK > 1 ? b[h].w : 0u);
+        bins[4 * h] = src.bin(a[h].x, b[h].x);
+        bins[4 * h + 1] = src.bin(a[h].y, b[h].y);
+        bins[4 * h + 2] = src.bin(a[h].z, b[h].z);
+        bins[4 * h + 3] = src.bin(a[h].w, b[h].w);
         if (Src::VAL) {
           val[4 * h] = v[h].x;
           val[4 * h + 1] = v[h].y;
@@ -230,8 +230,8 @@ tile_scatter_kernel(Src src, long long n, int ntiles, const long long* __restric
         bins[k] = NO_BIN;
         val[k] = 0;
         if (!full && i < n) {
-          bins[k] = src.bin(__ldcs(src.array(0) + i), NK > 1 ? __ldcs(src.array(1) + i) : 0u);
-          if (Src::VAL) val[k] = __ldcs(src.array(NK) + i);
+          bins[k] = src.bin(__ldcs(src.array(0) + i), __ldcs(src.array(1) + i));
+          if (Src::VAL) val[k] = __ldcs(src.array(2) + i);
         }
       }
     }
