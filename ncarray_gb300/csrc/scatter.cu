@@ -136,8 +136,8 @@ __device__ __forceinline__ void offsets_of(const ScatterArgs& a, long long i, lo
 
 // One grid-stride pass; SMEM: accumulate into the CTA's shared copy of dest.
 template <class D, bool SMEM>
-__global__ void __launch_bounds__(SMEM ? 1024 : THREADS) scatter_add_kernel(ScatterArgs a) {
-  const int nthr = SMEM ? (int)blockDim.x : THREADS;
+__global__ void __launch_bounds__(THREADS) scatter_add_kernel(ScatterArgs a) {
+  constexpr int nthr = THREADS;
   extern __shared__ __align__(16) unsigned char sm_raw[];
   D* priv = reinterpret_cast<D*>(sm_raw);
   if (SMEM) {
@@ -385,16 +385,24 @@ void launch(ScatterArgs& a, cudaStream_t s) {
     const long long flushed = (long long)sms * per_sm * a.dest_n;
     return sizeof(D) == 4 ? 2 * a.n >= flushed : 4 * a.n >= 3 * flushed;
   };
-  const int pct = bytes <= 48 * 1024 && pays(4) ? 4 : bytes <= 100 * 1024 && pays(2) ? 2 : 1;
-  const int pthreads = 1024 / pct;
-  const long long priv_ctas = (long long)sms * pct;
-  const bool smem = bytes <= SMEM_MAX_BYTES && pays(pct);
-  // few entries with many elements each: group sums too are better off in the copies
-  a.runs_direct = !(bytes <= 48 * 1024 && a.n >= 16ll * sms * a.dest_n);
   const int isz = (a.idx_dt == NCA_INT64 || a.idx_dt == NCA_UINT64) ? 8 : 4;
   const bool fast = a.nd == 1 && same_src<D>(a.src_dt) && a.dest_n < (1ll << 31) &&
                     a.istr[0] % isz == 0 && a.sstr[0] % (long long)sizeof(D) == 0 &&
                     (uintptr_t)a.idx % isz == 0 && (uintptr_t)a.src % sizeof(D) == 0;
+  int pct = bytes <= 48 * 1024 && pays(4) ? 4 : bytes <= 100 * 1024 && pays(2) ? 2 : 1;
+  bool smem = bytes <= SMEM_MAX_BYTES && pays(pct);
+  if (!fast) {
+    // the general kernel waits for its index arithmetic and groups always, so it
+    // needs the warps of 4 CTAs (one of 1024 threads: 2^24 elements of a transposed
+    // view into 50000 int32 entries 307 -> 459 us); 8-byte entries want many
+    // elements each (4 * 10^6 into 6000 float64 84 -> 93)
+    pct = 4;
+    smem = bytes <= 48 * 1024 && (sizeof(D) == 4 ? pays(4) && a.n >= (1 << 16) : a.n >= 16ll * sms * a.dest_n);
+  }
+  const int pthreads = 1024 / pct;
+  const long long priv_ctas = (long long)sms * pct;
+  // few entries with many elements each: group sums too are better off in the copies
+  a.runs_direct = !(bytes <= 48 * 1024 && a.n >= 16ll * sms * a.dest_n);
   // more shared memory than the default limit. Always the same value: the limit is
   // the kernel's on the device, and another thread may be launching it with more
   // than this call needs
@@ -424,8 +432,7 @@ void launch(ScatterArgs& a, cudaStream_t s) {
     }
   } else if (smem) {
     blocks = std::min(blocks, priv_ctas);
-    big((const void*)scatter_add_kernel<D, true>);
-    scatter_add_kernel<D, true><<<(unsigned)blocks, pthreads, (size_t)bytes, s>>>(a);
+    scatter_add_kernel<D, true><<<(unsigned)blocks, THREADS, (size_t)bytes, s>>>(a);
   } else {
     blocks = std::min(blocks, (long long)sms * 8);
     scatter_add_kernel<D, false><<<(unsigned)blocks, THREADS, 0, s>>>(a);
