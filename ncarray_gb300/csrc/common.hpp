@@ -108,12 +108,15 @@ struct StreamScratch {
 };
 
 // `n` arrival counters, all zero, for a kernel on stream `s` that leaves them
-// zero; null where the caller has to zero counters of its own. The marked ones
-// are for kernels that may leave any count: the launch's mark in the upper 44
-// bits, a count of up to 2^20 - 1 arrivals (a kernel's CTAs) in the lower 20.
+// zero; null where the caller has to zero counters of its own.
 uint32_t* arrival_counters(int64_t n, cudaStream_t s);
-unsigned long long* marked_counters(int64_t n, cudaStream_t s);
-uint64_t launch_mark();
+// The same for a kernel that may leave any count: counters that no earlier
+// launch has used since they were zeroed. The launch is made while `held` is.
+struct FreshCounters {
+  uint32_t* ptr = nullptr;
+  std::unique_lock<std::mutex> held;
+};
+FreshCounters fresh_counters(int64_t n, cudaStream_t s);
 
 // ---- chunk tables of the batched kernels --------------------------------------
 // Bytes per chunk: a CTA's share of the batch in whole slabs, between 128 and

@@ -1708,19 +1708,18 @@ static bool launch_staged_async(const Space& s, Spec sp, const Tape& tape, int q
   std::vector<uint64_t> w;
   fill_common_words(s, sp, tape, L, w);
   w[L.nsplit] = (uint64_t)G; w[L.chunk] = 0; w[L.keptn] = (uint64_t)KN; w[L.redn] = (uint64_t)RN;
-  // partial pieces of split units, and one marked arrival counter per unit
+  // partial pieces of split units, and one arrival counter per unit
   const int64_t slots = (G + U) * (int64_t)tp * QX;
   const size_t pbytes = sp.nred > 0 ? (size_t)slots * 8 * ((sp.has_sum ? 1 : 0) + (sp.has_max ? 2 : 0) + (sp.has_min ? 2 : 0)) : 0;
-  unsigned long long* cnt = sp.nred > 0 ? marked_counters(U, stream) : nullptr;
-  const size_t cbytes = sp.nred > 0 && !cnt ? ((size_t)U * 8 + 255) / 256 * 256 : 0;
+  const FreshCounters cnt = sp.nred > 0 ? fresh_counters(U, stream) : FreshCounters{};
+  const size_t cbytes = sp.nred > 0 && !cnt.ptr ? ((size_t)U * 4 + 255) / 256 * 256 : 0;
   StreamScratch part(pbytes + cbytes, stream);
   if (sp.nred > 0) {
     uint64_t* p = (uint64_t*)part.ptr;
     if (sp.has_sum) { w[L.psum] = (uint64_t)(uintptr_t)p; p += slots; }
     if (sp.has_max) { w[L.pmax] = (uint64_t)(uintptr_t)p; p += 2 * slots; }
     if (sp.has_min) { w[L.pmin] = (uint64_t)(uintptr_t)p; p += 2 * slots; }
-    w[L.aux] = (uint64_t)(uintptr_t)(cnt ? (void*)cnt : (void*)p);
-    w[L.chunk] = launch_mark();
+    w[L.aux] = (uint64_t)(uintptr_t)(cnt.ptr ? (void*)cnt.ptr : (void*)p);
     if (cbytes) check_cuda(cudaMemsetAsync(p, 0, cbytes, stream), "unit counters");
   }
   // the kernel takes the words and the first nmaps tensor maps

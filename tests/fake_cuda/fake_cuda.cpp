@@ -19,7 +19,7 @@
 namespace {
 struct Kernel {
   std::string name, defines;   // JSON members of the NCA_ constants
-  int chunk_word = -1;         // of a generated kernel: which argument word is its chunk
+  int aux_word = -1;           // of a generated kernel: which argument word is its counters' address
 };
 std::mutex mu;
 std::string log_text;
@@ -36,7 +36,7 @@ void record(const std::string& line) {
 void record_launch(const Kernel* k, dim3 g, dim3 b, size_t smem, const unsigned long long* words = nullptr) {
   record("{\"launch\": \"" + k->name + "\", \"grid\": [" + std::to_string(g.x) + ", " + std::to_string(g.y) + ", " +
          std::to_string(g.z) + "], \"block\": " + std::to_string(b.x) + ", \"smem\": " + std::to_string(smem) +
-         (words && k->chunk_word >= 0 ? ", \"chunk\": " + std::to_string(words[k->chunk_word]) : "") + ", \"consts\": {" + k->defines + "}}");
+         (words && k->aux_word >= 0 ? ", \"aux\": " + std::to_string(words[k->aux_word]) : "") + ", \"consts\": {" + k->defines + "}}");
 }
 // "#define NCA_NAME <integer>" lines of a source as JSON members
 std::string constants(const char* src) {
@@ -63,8 +63,8 @@ CUresult module_load(CUmodule* m, const void* image) {
 }
 CUresult module_function(CUfunction* f, CUmodule m, const char* name) {
   auto* k = new Kernel{name, constants(((std::string*)m)->c_str())};
-  const size_t at = k->defines.find("\"NCA_W_CHUNK\": ");
-  if (at != std::string::npos) k->chunk_word = atoi(k->defines.c_str() + at + 15);
+  const size_t at = k->defines.find("\"NCA_W_AUX\": ");
+  if (at != std::string::npos) k->aux_word = atoi(k->defines.c_str() + at + 13);
   *f = (CUfunction)k;
   return CUDA_SUCCESS;
 }
@@ -149,8 +149,8 @@ API cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaS
   return cudaSuccess;
 }
 API cudaError_t cudaFreeAsync(void* p, cudaStream_t) { free(p); return cudaSuccess; }
-API cudaError_t cudaMemsetAsync(void*, int, size_t n, cudaStream_t) {
-  record("{\"memset\": " + std::to_string(n) + "}");
+API cudaError_t cudaMemsetAsync(void* p, int, size_t n, cudaStream_t) {
+  record("{\"memset\": " + std::to_string(n) + ", \"at\": " + std::to_string((unsigned long long)p) + "}");
   return cudaSuccess;
 }
 API cudaError_t cudaMemcpyAsync(void*, const void*, size_t, cudaMemcpyKind, cudaStream_t) { return cudaSuccess; }

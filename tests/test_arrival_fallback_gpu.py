@@ -1,5 +1,5 @@
-"""Reductions whose last CTA merges, beyond the counters that a stream keeps: more sets of columns and more staged units than
-a block of 4096 counters, and more streams than there are blocks (64). Those zero counters of their own."""
+"""Reductions whose last CTA merges, beyond the counters that a stream keeps: more sets of columns than 4096, more staged
+units than 8192, and more streams than there are blocks (64). Those zero counters of their own."""
 import os
 import subprocess
 import sys

@@ -178,7 +178,7 @@ out = array((16384,), DType.float32)
 
 def launch():
     nca.DevExpr.leaf(x).evaluate(reductions=[(RedOp.SUM, 0)], red_out=[out])
-    return launches()
+    return [{k: v for k, v in c.items() if k != "aux"} for c in launches()]
 
 """
 
@@ -243,22 +243,33 @@ result = [schedule(h), open(sys.argv[2] + "/batch_tune_ws.txt").read()]
     assert fake_cuda.run(BATCH + "result = schedule(create())", old) != plain
 
 
-def test_launch_marks_leave_the_count_its_bits(built_lib, tmp_path):
-    """The marks of staged reductions' counters: another one for each launch, above 20 bits of count, so that one comes
-    again after 2^44 launches instead of 2^32."""
+def test_staged_launches_take_counters_that_are_still_zero(built_lib, tmp_path):
+    """Every launch counts in words that none before it has used since they were zeroed; no compare and swap, no memset of
+    its own. The block's memset comes when the next launch would not fit."""
     code = """
-t = array((64, 64, 128, 8), DType.int32).transpose(3, 1, 2, 0)
+t = array((64, 256, 128, 8), DType.int32).transpose(3, 1, 2, 0)
 e = nca.DevExpr.leaf(t) * np.int32(3)
 kept = [t.shape[d] for d in (0, 1, 3)]
 out, red = array(t.shape, e.expr_dtype), array(kept, e.expr_dtype)
-for _ in range(3):
+result = []
+for _ in range(60):
     e.evaluate(out, [(RedOp.MAX, 2)], [red])
-result = [[c["consts"]["NCA_KIND"], c["chunk"]] for c in launches()]
+    result += [["zero", c["at"], c["memset"]] if "memset" in c else ["count", c["aux"], c["consts"]["NCA_KIND"]]
+               for c in calls() if "launch" in c or "memset" in c]
 """
-    got = fake_cuda.run(code, tmp_path)
-    assert [k for k, _ in got] == [7] * 3
-    marks = [m for _, m in got]
-    assert all(m and m % 2**20 == 0 for m in marks) and len(set(marks)) == 3
+    events = fake_cuda.run(code, tmp_path)
+    first = events[0][1]
+    units = events[1][1] - first   # bytes that a launch takes
+    used, zeroed = set(), 0
+    for what, at, n in events:
+        if what == "zero":
+            assert (at, n) == (first, 4 * 8192)
+            used.clear()
+            zeroed += 1
+        else:
+            assert n == 7 and first <= at and at + units <= first + 4 * 8192 and at not in used
+            used.add(at)
+    assert units >= 4 * 256 and zeroed == 60 * units // (4 * 8192) - (60 * units % (4 * 8192) == 0)
 
 
 @pytest.mark.parametrize("name", ["nca_jit_selftest", "nca_jit_selftest_forms"])
