@@ -2263,6 +2263,9 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
     //     the second round ((256, 256, 1024) maximum over axis 1, 1024 sets: 48 ->
     //     58); from 16 on sums gain ((200, 777, 333) 50 -> 43), extremes do not
     //     ((128, 1200, 1024) maximum 95 -> 103)
+    //   operands strided along the kept dim take a load per element: (100, 1, 300,
+    //     100) transposed float32 times 3 plus another, stored with sum and maximum
+    //     over 300, 23 -> 29; odd rows, one element a lane anyway, gain
     //   float64 sums are bound by their pipe: (100, 60000) 20.6 -> 24.9, 4 operands
     //     of (1024, 4096) 48 -> 58; single arrays of few sets gain ((2000, 5000)
     //     41 -> 33). 8-bit sums beside extremes by their conversions, once long:
@@ -2271,15 +2274,19 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
     const int64_t m = cdiv(RN, R);   // rows of a lane
     const bool f64 = arith_dtype(tape.compute_dtype) == NCA_FLOAT64;
     const bool single = (has_sum ? 1 : 0) + (has_max ? 1 : 0) + (has_min ? 1 : 0) == 1;
+    bool apart = false;   // an operand whose neighbours along the kept dim are not adjacent
+    for (int k = 0; k < nops; ++k)
+      if (s.ops[k].st[s.nd - 1] != 0 && s.ops[k].st[s.nd - 1] != dtinfo(s.ops[k].dtype).size) apart = true;
     if (out) {
-      sp.k4g = !fill || (m >= 5 && nops <= (f64 ? 6 : 12)) ? 1 : 0;
+      sp.k4g = !fill || (m >= 5 && nops <= (f64 ? 6 : 12) && !(apart && sp.vec > 1)) ? 1 : 0;
       if (fill && f64 && sp.k4g) sp.unroll = unroll = 2;
     } else {
       int widest = 1;
       for (int k = 0; k < nops; ++k) widest = std::max(widest, dtinfo(s.ops[k].dtype).size);
       const bool filled = m >= 5 && (m <= 8 || 5 * cdiv(m, 8) * 8 <= 7 * m);
       const bool few = nset <= 4 * (int64_t)sms, many = nset >= 16 * (int64_t)sms;
-      sp.k4g = fill && nops <= 12 && (few ? filled || !single : many && has_sum && filled) ? 1 : 0;
+      sp.k4g = fill && !(apart && sp.vec > 1) && nops <= 12 &&
+               (few ? filled || !(single || apart) : many && has_sum && filled) ? 1 : 0;
       if (f64 && has_sum && single && (nops > 1 || m < 16 || (few && nset > 2 * (int64_t)sms))) sp.k4g = 0;
       if (widest == 1 && !single && RN >= 4096) sp.k4g = 0;
       if (sp.k4g && few) {

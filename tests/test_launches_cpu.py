@@ -103,8 +103,8 @@ for n in (2, 3, 4, 6, 12, 24, 48):
 
 
 OUTER = """
-def outer(shape, axis, dtype, nops=1, ops=(RedOp.SUM,), stored=False):
-    xs = [array(shape, dtype) for _ in range(nops)]
+def outer(shape, axis, dtype, nops=1, ops=(RedOp.SUM,), stored=False, step=1):
+    xs = [array((*shape[:-1], shape[-1] * step), dtype)[..., ::step] for _ in range(nops)]
     e = nca.DevExpr.leaf(xs[0])
     for x in xs[1:]:
         e = e + x
@@ -132,6 +132,7 @@ result = {
     "rows": [outer((n, 1000000), 0, F) for n in (5, 16, 20, 32, 33, 64, 100)],
     "stored_rows": [outer((n, 100000), 0, F, stored=True) for n in (5, 16, 20, 33)],
     "two": [outer((n, 5000), 0, F, ops=(RedOp.SUM, RedOp.MAX)) for n in (5, 33)],
+    "strided": [outer((256, w), 0, F, stored=st, step=2) for w in (1000, 1001) for st in (False, True)],
     "sum64": [outer(s, 0, D, n) for s, n in (((2000, 5000), 1), ((2000, 5000), 2), ((100, 60000), 1), ((33, 1000000), 1))],
 }
 """
@@ -142,7 +143,7 @@ fake.fake_resident(3)
 result = [outer((1200, 4 * 64 * n), 0, DType.float32) for n in (400, 456, 457, 500)]
 """, tmp_path)
     assert got == {"stored": [8, 8, 8, 0, 0, 0], "reduced": [8, 8, 8, 0, 0, 0], "stored64": [2, 2, 0, 0],
-                   "rows": [0, 0, 8, 8, 0, 8, 8], "stored_rows": [0, 0, 8, 8], "two": [8, 8], "sum64": [8, 0, 0, 0],
+                   "rows": [0, 0, 8, 8, 0, 8, 8], "stored_rows": [0, 0, 8, 8], "two": [8, 8], "strided": [0, 0, 8, 8], "sum64": [8, 0, 0, 0],
                    "round": [8, 8, 0, 0]}
 
 
