@@ -2270,6 +2270,7 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
     //     of (1024, 4096) 48 -> 58; single arrays of few sets gain ((2000, 5000)
     //     41 -> 33). 8-bit sums beside extremes by their conversions, once long:
     //     (20000, 500) 33 -> 40
+    CUfunction together = nullptr;
     const bool fill = tps < 0;
     const int64_t m = cdiv(RN, R);   // rows of a lane
     const bool f64 = arith_dtype(tape.compute_dtype) == NCA_FLOAT64;
@@ -2291,7 +2292,8 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
       if (widest == 1 && !single && RN >= 4096) sp.k4g = 0;
       if (sp.k4g && few) {
         sp.lastcta = lastcta;
-        if (nset > (int64_t)sms * resident_ctas(kernel_for(sp, tape))) sp.k4g = 0;
+        together = kernel_for(sp, tape);
+        if (nset > (int64_t)sms * resident_ctas(together)) sp.k4g = 0;
       }
     }
     if (fill) tps = RN <= 256 ? 512 : 1024;
@@ -2354,7 +2356,7 @@ bool expr_reduce(const Tape& tape, const nca_view* ops, int nops, const nca_view
       // at least 16 sets of columns, since the merge walks the splits
       // ((16384, 1024) bfloat16, 152 splits: 30 us, 190: 36)
       sp.lastcta = lastcta;
-      fn = kernel_for(sp, tape);
+      fn = together ? together : kernel_for(sp, tape);
       const int64_t fit = (int64_t)sms * resident_ctas(fn) / nset, trip = (int64_t)unroll * R;
       S = std::max<int64_t>(1, std::min<int64_t>(fit, nset >= 16 ? std::max<int64_t>(S, RN / (2 * trip)) : S));
       C = cdiv(cdiv(RN, trip), S) * trip;
