@@ -710,8 +710,8 @@ void launch3_as(const Grid3& src, const Grid3& dst, const Weights<float>& W, cud
 // 156; (8, 2048, 2048) 135, 123 / 160, 207; (16, 2048, 2048) 261, 183 / 302, 307;
 // (8, 8, 100000) 49, 103 / 68, 89; (512, 512, 32) 67, 70 / 92, 107; (64, 64, 64)
 // 25, 14 / 31, 12; (512, 512, 512) 511, 300 / 510, 481. Of 74 grids measured the
-// rule takes the slower form for four, by 5 % or less in all but one
-// ((512, 512, 132) with 27 points keeps single steps: 221 against 209).
+// rule takes the slower form for three, by 5 % at most ((512, 512, 132) with 27
+// points keeps single steps: 221 against 209).
 bool three_pays(const Grid3& g, int mode, int sms, int tile, int zt1) {
   const bool star = mode == 1;
   int zt = g.nz;
@@ -775,7 +775,7 @@ void run(const nca_view* a, const nca_view* b, const double* w27, double dt, int
 namespace {
 // Arrival counters of kernels whose last CTA merges the partial results, one
 // block of them per stream (see stream_words). Zero when the module loads.
-constexpr int ARR_STREAMS = 64, ARR_N = 4096, FRESH_N = 8192;
+constexpr int ARR_STREAMS = 64, ARR_N = 4096, FRESH_N = 16384;
 __device__ uint32_t g_arrivals[ARR_STREAMS][ARR_N];
 __device__ uint32_t g_fresh[ARR_STREAMS][FRESH_N];
 }  // namespace

@@ -1,5 +1,5 @@
 """Reductions whose last CTA merges, beyond the counters that a stream keeps: more sets of columns than 4096, more staged
-units than 8192, and more streams than there are blocks (64). Those zero counters of their own."""
+units than 16384, and more streams than there are blocks (64). Those zero counters of their own."""
 import os
 import subprocess
 import sys
@@ -29,7 +29,7 @@ def test_more_sets_than_counters(cuda, monkeypatch):
 
 
 def test_more_staged_units_than_counters(cuda):
-    h = np.random.default_rng(SEED + 461).integers(-9, 9, (64, 4200, 40, 8)).astype(np.int32)   # (p, b, r, q)
+    h = np.random.default_rng(SEED + 461).integers(-9, 9, (64, 8200, 24, 8)).astype(np.int32)   # (p, b, r, q)
     t = nca.NCDevArray.from_host(h).transpose(3, 1, 2, 0)
     with nca.lazy_mode():
         e = t * np.int32(3)

@@ -253,7 +253,7 @@ e = nca.DevExpr.leaf(t) * np.int32(3)
 kept = [t.shape[d] for d in (0, 1, 3)]
 out, red = array(t.shape, e.expr_dtype), array(kept, e.expr_dtype)
 result = []
-for _ in range(60):
+for _ in range(120):
     e.evaluate(out, [(RedOp.MAX, 2)], [red])
     result += [["zero", c["at"], c["memset"]] if "memset" in c else ["count", c["aux"], c["consts"]["NCA_KIND"]]
                for c in calls() if "launch" in c or "memset" in c]
@@ -264,13 +264,13 @@ for _ in range(60):
     used, zeroed = set(), 0
     for what, at, n in events:
         if what == "zero":
-            assert (at, n) == (first, 4 * 8192)
+            assert (at, n) == (first, 4 * 16384)
             used.clear()
             zeroed += 1
         else:
-            assert n == 7 and first <= at and at + units <= first + 4 * 8192 and at not in used
+            assert n == 7 and first <= at and at + units <= first + 4 * 16384 and at not in used
             used.add(at)
-    assert units >= 4 * 256 and zeroed == 60 * units // (4 * 8192) - (60 * units % (4 * 8192) == 0)
+    assert units >= 4 * 256 and zeroed == 120 * units // (4 * 16384) - (120 * units % (4 * 16384) == 0)
 
 
 @pytest.mark.parametrize("name", ["nca_jit_selftest", "nca_jit_selftest_forms"])
