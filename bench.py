@@ -739,6 +739,15 @@ def profile_op(torch, nca, op: str, steps: int) -> None:
         b = nca.NCDevArray((512, 512, 512), nca.DType.float32)
         a._buf.view(torch.float32).normal_()
         fn = lambda: st.apply(a, b)  # noqa: E731
+    elif op == "c3-7-four-small":
+        # four 7-point iterations in one call (a three-step pass and a single step) on a
+        # (256, 512, 512) float32 grid (two buffers of 268 MB, above L2)
+        from ncarray_gb300.stencil import Stencil3D, laplacian7
+        st = Stencil3D(laplacian7(), 0.1)
+        a = nca.NCDevArray((256, 512, 512), nca.DType.float32)
+        b = nca.NCDevArray((256, 512, 512), nca.DType.float32)
+        a._buf.view(torch.float32).normal_()
+        fn = lambda: st.iterate(a, b, 4)  # noqa: E731
     elif op == "c1":
         rng = np.random.default_rng(SEED)
         da, db, dc = (nca.NCDevArray.from_host(rng.uniform(-1, 1, (128, 128, 128))) for _ in range(3))

@@ -257,12 +257,12 @@ struct Sum3 {
 // tiles one has pieces from many CTAs, and a loop over them is a chain of load
 // latency (CG = 8 from 8 pieces a tile on: 64 x 64 bins, 2^20 weighted points 54
 // us a call with CG = 4, 48 with 8; 1024 x 1024 bins have 2-3 pieces a tile,
-// CG = 1). The sharing CTAs come from the prefix pass and the weights are sums of three floats (Sum3):
-// 64-bit divisions and float64 adds and conversions per bin were most of the
-// pass (50-65 us for 1024 x 1024 weighted bins, 20-22 with pairs of floats;
-// with three a call takes the same time within 1 us). The output's old value is
-// one more term: 2^20 points added to 2048 x 2048 bins 160 -> 134 us a call
-// without float64 arithmetic for it.
+// CG = 1). The sharing CTAs come from the prefix pass and the weights are sums
+// of three floats (Sum3): 64-bit divisions and float64 adds and conversions per
+// bin were most of the pass (50-65 us for 1024 x 1024 weighted bins, 20-22 with
+// pairs of floats; with three a call takes the same time within 1 us). The
+// output's old value is one more term: 2^20 points added to 2048 x 2048 bins
+// 160 -> 134 us a call without float64 arithmetic for it.
 template <bool WEIGHTED, int CG>
 __global__ void __launch_bounds__(THREADS)
 tile_combine_kernel(long long nbins, int G, const long long* __restrict__ PV,
