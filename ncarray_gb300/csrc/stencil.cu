@@ -702,16 +702,19 @@ void launch3_as(const Grid3& src, const Grid3& dst, const Weights<float>& W, cud
 // Whether a three-step pass is shorter than three single steps: both are
 // estimated, in us. A pass takes its planes end to end, 0.93 us each for 7
 // points and 0.82 for 27 (1.13 and 0.94 where only one round of CTAs runs, which
-// nothing overlaps). A single step takes the time of one CTA's march, or of all
-// CTAs (several an SM), or of the bytes, whichever is longest. What tiles of 120
-// columns and 36 or 18 rows waste on a narrow grid, and the 10 extra planes of
-// a chunk on a flat one, decides: three steps against one pass, 7 points / 27,
+// nothing overlaps). A single step takes a start, a CTA's march and what the
+// CTAs of an SM issue together, or the bytes if those take longer. What tiles of
+// 120 columns and 36 or 18 rows waste on a narrow grid, and the 10 extra planes
+// of a chunk on a flat one, decides: three steps against one pass, 7 points / 27,
 // (1, 2048, 2048) 43 against 74 / 55 against 129; (4, 2048, 2048) 80, 92 / 103,
 // 156; (8, 2048, 2048) 135, 123 / 160, 207; (16, 2048, 2048) 261, 183 / 302, 307;
-// (8, 8, 100000) 49, 103 / 68, 89; (512, 512, 32) 67, 70 / 92, 107; (64, 64, 64)
-// 25, 14 / 31, 12; (512, 512, 512) 511, 300 / 510, 481. Of 74 grids measured the
-// rule takes the slower form for three, by 5 % at most ((512, 512, 132) with 27
-// points keeps single steps: 221 against 209).
+// (8, 8, 100000) 49, 103 / 68, 89; (29, 437, 340) 31, 23 / 37, 25; (64, 64, 64)
+// 25, 14 / 31, 12; (512, 512, 512) 511, 300 / 510, 481. The single step's numbers
+// are fitted to 170 grids of 1 to 512 planes, both weights: its estimate is off
+// by 5 % on average, and the rule takes the slower form on nine thin grids, by
+// 9 % at most ((3, 16, 148) 13.4 against 12.3), costing 0.2 % on average. With
+// the march and the issue taken as the longer of the two, without the start, 47
+// of the 340 took a form slower by more than 3 %, up to 1.5 times.
 bool three_pays(const Grid3& g, int mode, int sms, int tile, int zt1) {
   const bool star = mode == 1;
   int zt = g.nz;
@@ -721,12 +724,16 @@ bool three_pays(const Grid3& g, int mode, int sms, int tile, int zt1) {
   const int d = std::min(zt1, g.nz) + 2;
   const int64_t n = (int64_t)((g.nx + kTiles[tile][0] - 1) / kTiles[tile][0]) *
                     ((g.ny + kTiles[tile][1] - 1) / kTiles[tile][1]) * ((g.nz + zt1 - 1) / zt1);
-  const bool few = n <= 4 * (int64_t)sms;
-  const double r = few ? (double)((n + sms - 1) / sms) : (double)n / sms;
-  const double march = star ? 2.6 + 0.35 * d : 2.9 + 0.4 * d;
-  const double issue = (star ? (few ? 0.165 : 0.155) : (few ? 0.225 : 0.187)) * d * r;
-  const double bytes = (double)g.nx * g.ny * g.nz * 8.0 / 6.7e6;
-  return pass < 3.0 * std::max(march, std::max(issue, bytes));
+  double work;
+  if (n <= 4 * (int64_t)sms) {   // every CTA at once
+    const double r = (double)((n + sms - 1) / sms);
+    work = star ? 3.1 + 0.2 * d + 0.1 * d * r : 3.1 + 0.25 * d + 0.155 * d * r;
+  } else {
+    const double r = (double)n / sms;
+    work = star ? 2.5 + 0.16 * d * r : 4.7 + 0.19 * d * r;
+  }
+  const double bytes = (star ? 1.5 : 2.0) + (double)g.nx * g.ny * g.nz * 8.0 / 6.7e6;
+  return pass < 3.0 * std::max(work, bytes);
 }
 
 void launch3(const Grid3& src, const Grid3& dst, const Weights<float>& W, int mode, cudaStream_t s) {

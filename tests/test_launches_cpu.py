@@ -67,6 +67,23 @@ for points, w in ((7, laplacian7()), (27, laplacian27())):
         assert three == want, (points, shape)
 
 
+def test_three_step_stencil_on_grids_of_one_round(built_lib, tmp_path):
+    """Grids whose CTAs all run at once, where a single step's start and march are most of its time: a pass took 0.67 to
+    0.95 of three single steps; thin ones, where it takes longer, keep single steps."""
+    code = """
+from ncarray_gb300.stencil import Stencil3D, laplacian7, laplacian27
+result = []
+for points, w in ((7, laplacian7()), (27, laplacian27())):
+    for shape in ((29, 437, 340), (43, 408, 168), (57, 445, 136), (100, 208, 272), (34, 304, 136), (192, 193, 296), (512, 512, 132),
+                  (1, 290, 1452), (2, 1024, 1024)):
+        a, b = array(shape, DType.float32), array(shape, DType.float32)
+        Stencil3D(w, 0.1).iterate(a, b, 4)
+        result.append([points, shape, ["tma3" in c["launch"] for c in launches()]])
+"""
+    for points, shape, three in fake_cuda.run(code, tmp_path):
+        assert three == ([True, False] if shape[0] > 3 else [False] * 4), (points, shape)
+
+
 def test_weighted_histogram_uses_every_cta(built_lib, tmp_path):
     """2^20 weighted points accumulate on one CTA per resident slot even where the bins outnumber a CTA's records: points
     that crowd into one bin are as many serial adds as a CTA has."""
